@@ -236,14 +236,11 @@ toed_status toed_detect_noalloc(const toed_image* image, const toed_params* para
  * the launch -- another host thread that waits for the whole device in that
  * moment (cudaDeviceSynchronize, cudaFree) can hold those copies back until
  * the wait gives up (TOED_ERR_TIMEOUT), so serialise such calls; with
- * CUDA_LAUNCH_BLOCKING or under a profiler this flow is not used.  With
- * chunks == 1 no copy at all (the kernel reads them in place through their
- * device mapping).  Pageable
+ * CUDA_LAUNCH_BLOCKING or under a profiler this flow is not used.  Pageable
  * images, or more than 64: one launch per group (streams of the context,
- * ordered by events).  Page-locked
- * output buffers (edgels, count,
- * grid_index) are written by the detection's ordering pass directly through
- * their device mapping; pageable ones are filled by copies per group once its
+ * ordered by events).  Page-locked output buffers (edgels, count, grid_index)
+ * are written by a kernel through their device mapping once the lists are
+ * complete; pageable ones are filled by copies per group once its
  * counts are read back.  Synchronous: returns when every count and list is in
  * host memory.  Device staging is kept in the context and grows on demand.
  * Page-locked image buffers give full copy speed.  Returns
@@ -277,22 +274,21 @@ toed_status toed_write_edgels_txt(const char* path, const void* edgels, int dtyp
 
 /* Launch-shape autotuning (no counterpart in the reference, whose GPU path
  * has one fixed launch shape).  toed_autotune times each candidate -- strip
- * height 14, 30, 62, 126, 254, 510 or 1022 rows, input rows staged by TMA, by
- * per-thread async copies or by plain loads -- on the caller's batch with CUDA
- * events, `reps` timed runs
+ * height 16k - 2 rows for twelve k from 1 to 64, input rows staged by TMA or
+ * by loads -- on the caller's batch with CUDA events, `reps` timed runs
  * after one untimed run each, keeps the fastest in the context for this
  * radius, precision and launch size class -- floor(log2(pixels)) of each
  * launch of the batch (64 images at most per launch) -- and returns it; later
  * launches of the same class use it, launches of other classes keep the
  * built-in heuristic.
- * It is synchronous, runs the detection 21 * (reps + 1) times (the outputs hold
+ * It is synchronous, runs the detection 24 * (reps + 1) times (the outputs hold
  * the last run; every candidate gives the same result bit for bit) and is
  * refused under stream capture.  toed_set_tuning installs a shape for every
  * size class (NULL restores the built-in heuristic). */
 typedef struct toed_tuning {
     int strip_rows;  /* 16k - 2 for k in 1, 2, 4, ..., 64 */
-    int staging;     /* input row staging: 1 TMA (when the image allows it), 2 per-thread async
-                        copies two steps ahead (float32 images), 0 plain loads */
+    int staging;     /* input row staging: 1 TMA (float32 images whose rows are 16-byte aligned),
+                        0 or 2 loads prefetched a step ahead in registers */
     float ms;        /* measured time of one detection of the batch (autotune output) */
 } toed_tuning;
 

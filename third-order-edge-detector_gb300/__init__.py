@@ -258,7 +258,7 @@ class HostBatch:
 
     def run(self, params: toed_params, chunks=None, stream=None):
         """chunks: copy groups (None: one image per group, the fastest for
-        page-locked images; 1: page-locked images read in place)."""
+        page-locked images)."""
         det = self.det
         if chunks is None:
             chunks = len(self.images)
@@ -366,7 +366,8 @@ class Detector:
 
     def set_tuning(self, params: toed_params, strip_rows=None, staging="tma"):
         """Install a launch shape (strip_rows None: the built-in heuristic);
-        staging: "tma", "async" or "plain" (True / False mean "tma" / "plain")."""
+        staging: "tma", or "async" / "plain" for loads (True / False mean "tma" /
+        "plain")."""
         if isinstance(staging, bool):
             staging = "tma" if staging else "plain"
         t = toed_tuning(int(strip_rows), _STAGING_NAMES.index(staging), 0.0) if strip_rows is not None else None

@@ -18,35 +18,34 @@
 #include "toed_internal.h"
 
 namespace toed {
-DetectEntry detect_entry_r1(bool, bool, bool);
-DetectEntry detect_entry_r2(bool, bool, bool);
-DetectEntry detect_entry_r3(bool, bool, bool);
-DetectEntry detect_entry_r4(bool, bool, bool);
-DetectEntry detect_entry_r5(bool, bool, bool);
-DetectEntry detect_entry_r6(bool, bool, bool);
-DetectEntry detect_entry_r7(bool, bool, bool);
-DetectEntry detect_entry_r8(bool, bool, bool);
-DetectEntry detect_entry_r9(bool, bool, bool);
-DetectEntry detect_entry_r10(bool, bool, bool);
-DetectEntry detect_entry_r11(bool, bool, bool);
-DetectEntry detect_entry_r12(bool, bool, bool);
+DetectEntry detect_entry_r1(bool);
+DetectEntry detect_entry_r2(bool);
+DetectEntry detect_entry_r3(bool);
+DetectEntry detect_entry_r4(bool);
+DetectEntry detect_entry_r5(bool);
+DetectEntry detect_entry_r6(bool);
+DetectEntry detect_entry_r7(bool);
+DetectEntry detect_entry_r8(bool);
+DetectEntry detect_entry_r9(bool);
+DetectEntry detect_entry_r10(bool);
+DetectEntry detect_entry_r11(bool);
+DetectEntry detect_entry_r12(bool);
 
-DetectEntry detect_entry(int r, bool hyb, bool async, bool nmsto)
+DetectEntry detect_entry(int r, bool nmsto)
 {
-    if (nmsto) async = false;
     switch (r) {
-    case 1: return detect_entry_r1(hyb, async, nmsto);
-    case 2: return detect_entry_r2(hyb, async, nmsto);
-    case 3: return detect_entry_r3(hyb, async, nmsto);
-    case 4: return detect_entry_r4(hyb, async, nmsto);
-    case 5: return detect_entry_r5(hyb, async, nmsto);
-    case 6: return detect_entry_r6(hyb, async, nmsto);
-    case 7: return detect_entry_r7(hyb, async, nmsto);
-    case 8: return detect_entry_r8(hyb, async, nmsto);
-    case 9: return detect_entry_r9(hyb, async, nmsto);
-    case 10: return detect_entry_r10(hyb, async, nmsto);
-    case 11: return detect_entry_r11(hyb, async, nmsto);
-    case 12: return detect_entry_r12(hyb, async, nmsto);
+    case 1: return detect_entry_r1(nmsto);
+    case 2: return detect_entry_r2(nmsto);
+    case 3: return detect_entry_r3(nmsto);
+    case 4: return detect_entry_r4(nmsto);
+    case 5: return detect_entry_r5(nmsto);
+    case 6: return detect_entry_r6(nmsto);
+    case 7: return detect_entry_r7(nmsto);
+    case 8: return detect_entry_r8(nmsto);
+    case 9: return detect_entry_r9(nmsto);
+    case 10: return detect_entry_r10(nmsto);
+    case 11: return detect_entry_r11(nmsto);
+    case 12: return detect_entry_r12(nmsto);
     default: return DetectEntry{nullptr, 0};
     }
 }
@@ -79,6 +78,12 @@ void make_taps(double sigma, int r, TapBlock* tb)
         for (int k = 0; k < kMaxTaps; ++k) tb->v[f][k] = (float)d.v[f][k];
 }
 
+void make_ytap(const TapBlock& t, float2 (*ytap)[kMaxTaps])
+{
+    for (int v = 0; v < 2; ++v)
+        for (int k = 0; k < kMaxTaps; ++k) ytap[v][k] = make_float2(t.v[4 * v + 1][k], t.v[4 * v][k]);
+}
+
 static PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
 {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
@@ -97,28 +102,16 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
 void encode_rows_map(CUtensorMap* m, DetImage& d, int r)
 {
     d.tma = 0;
-    d.tma_align = 1;
-    d.tma_boxw = 0;
-    const int esz = (d.dtype == TOED_U8) ? 1 : 4;
-    const int align = 16 / esz;
-    const int nin = kExt + 2 * r + 2;
-    const int boxw = (nin + align - 1 + align - 1) / align * align;
     auto fn = encode_fn();
-    if (!fn || (reinterpret_cast<uintptr_t>(d.src) & 15u) != 0 || ((long long)d.pitch * esz) % 16 != 0 ||
-        boxw * esz > kRawRowBytes)
-        return;
+    if (!fn || d.dtype != TOED_F32 || (reinterpret_cast<uintptr_t>(d.src) & 15u) != 0 || d.pitch % 4 != 0) return;
     const cuuint64_t dims[2] = {(cuuint64_t)d.W, (cuuint64_t)d.H};
-    const cuuint64_t strides[1] = {(cuuint64_t)d.pitch * esz};
-    const cuuint32_t box[2] = {(cuuint32_t)boxw, (cuuint32_t)kStepRows};
+    const cuuint64_t strides[1] = {(cuuint64_t)d.pitch * sizeof(float)};
+    const cuuint32_t box[2] = {(cuuint32_t)staged_width(r), (cuuint32_t)kStepRows};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult res = fn(m, esz == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
-                            const_cast<void*>(d.src), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (res != CUDA_SUCCESS) return;
-    d.tma = 1;
-    d.tma_align = align;
-    d.tma_boxw = boxw;
+    const CUresult res = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(d.src), dims, strides, box, estr,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    d.tma = res == CUDA_SUCCESS;
 }
 
 }  // namespace toed
@@ -146,7 +139,7 @@ static thread_local std::string g_last_cuda_error;
 struct toed_ctx {
     int device = 0;
     int num_sms = 0;
-    int* words = nullptr;  // kWords: [0] queue [1] cursor [2] flags [3] refine-list length [4] debug
+    int* words = nullptr;  // kWords: [0] queue [1] cursor [2] flags [3] tile ticket [4] debug
     double4_32a* staging = nullptr;
     int* staging_idx = nullptr;
     long long staging_cap = 0;
@@ -156,8 +149,10 @@ struct toed_ctx {
     long long tile_cap = 0;
     long long* img_base = nullptr;
     int img_cap = 0;
-    int4* refine = nullptr;  // orientation recomputation list
-    long long refine_cap = 0;
+    int* seg_dst = nullptr;
+    long long dst_cap = 0;
+    unsigned long long* tile_state = nullptr;  // the scan's tiles
+    long long state_cap = 0;
     float2* dir = nullptr;
     int* eid = nullptr;
     int* win = nullptr;
@@ -168,7 +163,8 @@ struct toed_ctx {
     long long keep_cap = 0;
     double* sp_work = nullptr;  // TO correction at interp_n > 0: maps resized onto the work grid
     long long sp_work_cap = 0;
-    int blocks_per_sm[TOED_MAX_RADIUS + 1][2][3] = {};  // [radius][hybrid][TMA/plain, async, corrected normal]
+    int blocks_per_sm[TOED_MAX_RADIUS + 1][2] = {};  // [radius][corrected normal]
+    bool edgels_ready[TOED_MAX_RADIUS + 1] = {};     // the edgel kernel's attributes are set
     // launch shape chosen by toed_autotune per (radius, precision, size class of
     // the launch: floor(log2(pixels))); strip_rows 0 = heuristic
     toed_tuning tune[TOED_MAX_RADIUS + 1][2][kSizeClasses] = {};
@@ -270,7 +266,8 @@ toed_status toed_destroy(toed_ctx* c)
     cudaFree(c->seg);
     cudaFree(c->tile_sum);
     cudaFree(c->img_base);
-    cudaFree(c->refine);
+    cudaFree(c->tile_state);
+    cudaFree(c->seg_dst);
     cudaFree(c->dir);
     cudaFree(c->eid);
     cudaFree(c->win);
@@ -320,10 +317,10 @@ static toed_status ensure_scratch(toed_ctx* c, long long staging, long long segs
     long long sc2 = c->staging_cap;
     if ((st = grow(&c->staging_idx, &sc2, staging, stream)) != TOED_OK) return st;
     c->staging_cap = std::min(sc, sc2);
-    // one entry per 64 staged edgels (about 1 in 5000 is listed on noisy images)
-    if ((st = grow(&c->refine, &c->refine_cap, staging / 64 + 1024, stream)) != TOED_OK) return st;
     if ((st = grow(&c->seg, &c->seg_cap, segs, stream)) != TOED_OK) return st;
+    if ((st = grow(&c->seg_dst, &c->dst_cap, segs, stream)) != TOED_OK) return st;
     if ((st = grow(&c->tile_sum, &c->tile_cap, tiles, stream)) != TOED_OK) return st;
+    if ((st = grow(&c->tile_state, &c->state_cap, tiles, stream)) != TOED_OK) return st;
     long long ic = c->img_cap;
     if ((st = grow(&c->img_base, &ic, (long long)imgs, stream)) != TOED_OK) return st;
     c->img_cap = (int)ic;
@@ -338,11 +335,11 @@ extern "C" toed_status toed_reserve(toed_ctx* c, long long max_pixels, long long
     TOED_CU(cudaSetDevice(c->device));
     // segments: 2 rows per pixel row x ceil(W/30) strip columns, bounded by pixels/15 + tiles of padding
     const int imgs = std::min(std::max(max_images, 1), kBatchMax);
-    const long long segs = max_pixels / 15 + 2LL * 4096 + (long long)imgs * kSegTile;
+    const long long segs = max_pixels / 15 + 2LL * 4096 + (long long)imgs * kScanTileMax;
     const long long tiles = segs / kSegTile + imgs + 1;
     std::lock_guard<std::mutex> lk(c->mu);
-    // staging slack: one reservation block per resident CTA (at most 4 per SM)
-    const long long slack = 4LL * c->num_sms * kStageBlk;
+    // staging slack: one reservation block per resident warp (at most 4 CTAs per SM)
+    const long long slack = 4LL * c->num_sms * (kThreads / 32) * kStageBlk;
     toed_status st = ensure_scratch(c, std::max(max_edgels, 1LL) + slack, segs, tiles, imgs, nullptr);
     cudaSetDevice(prev);
     return st;
@@ -392,44 +389,58 @@ static int plan_strip_rows(const toed_image* images, int n, long long resident)
     return kStepRows - 2;
 }
 
-// plain_loads: never stage input rows by TMA (images read in place from
-// page-locked host memory through their device mapping): float32 rows by
-// per-thread async copies one step ahead, uint8 rows by plain loads
+// Segments per tile of the scan: few tiles to look back over on a small
+// launch (25 on a 752 x 480 image; at 64 segments a tile its 390 took 10 us),
+// one wave of them on a large one.
+static int plan_seg_tile(long long nseg) { return nseg > 1024LL * kSegTile ? kScanTileMax : kSegTile; }
+
+// Image rows of an edgel-kernel tile: as tall as possible (a tile's pixels
+// include 2r + 2 rows of halo) while every SM still gets several tiles.
+static int plan_ed_rows(const toed_image* images, int n, int num_sms)
+{
+    long long rows = 0;  // strip rows of the launch
+    for (int i = 0; i < n; ++i) rows += (long long)((images[i].width + kInner - 1) / kInner) * images[i].height;
+    int t = kEdRowsMax;
+    while (t > 16 && rows < (long long)t * 8 * num_sms) t /= 2;
+    return t;
+}
+
 // wait_slot (optional, per image): 0, or g > 0 when the copy engine is still
 // bringing the image in and c->hb_ready[g - 1] == c->hb_epoch marks its arrival
 static toed_status detect_chunk(toed_ctx* c, const toed_image* images, int n, const toed_params* prm,
                                 int r, bool first_chunk, cudaStream_t stream, const toed_tuning* force = nullptr,
-                                bool plain_loads = false, const int* wait_slot = nullptr)
+                                const int* wait_slot = nullptr)
 {
     const bool hyb = prm->precision != TOED_FP32;
     const bool nmsto = prm->nms_direction == TOED_NMS_TO_NORMAL;
     const toed_tuning& tuned = c->tune[r][hyb ? 1 : 0][size_class(images, n)];
     const toed_tuning* use = force ? force : (tuned.strip_rows > 0 ? &tuned : nullptr);
-    // async row staging: images read in place from host memory, or the tuned
-    // shape asks for it (the corrected-normal kernel stages rows by TMA or
-    // plain loads only)
-    const bool async_rows = !nmsto && (plain_loads || (use && use->staging == 2));
-    DetectEntry ent = detect_entry(r, hyb, async_rows, nmsto);
+    DetectEntry ent = detect_entry(r, nmsto);
     if (!ent.func) return TOED_ERR_UNSUPPORTED;
-    int& bps = c->blocks_per_sm[r][hyb ? 1 : 0][nmsto ? 2 : (async_rows ? 1 : 0)];
+    int& bps = c->blocks_per_sm[r][nmsto ? 1 : 0];
     if (bps == 0) {
         TOED_CU(cudaFuncSetAttribute(ent.func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ent.smem));
         TOED_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, ent.func, kThreads, ent.smem));
         if (bps <= 0) return TOED_ERR_UNSUPPORTED;
     }
     const long long resident = (long long)bps * c->num_sms;
+    if (!c->edgels_ready[r]) {
+        TOED_CU(prepare_edgels(r));
+        c->edgels_ready[r] = true;
+    }
 
     BatchParams* p = new BatchParams();
     std::unique_ptr<BatchParams> guard(p);
     // the taps of the last (sigma, radius), kept in the context (a few hundred exp per call otherwise)
     if (c->tap_sigma != prm->sigma || c->tap_r != r) {
-        make_taps((double)prm->sigma, r, &c->taps);
         make_taps64((double)prm->sigma, r, &c->taps64);
+        make_taps((double)prm->sigma, r, &c->taps);
         c->tap_sigma = prm->sigma;
         c->tap_r = r;
     }
     p->taps = c->taps;
     p->taps64 = c->taps64;
+    make_ytap(c->taps, p->ytap);
     p->thr = prm->threshold;
     p->thr2 = prm->threshold < 0.f ? -1.f : prm->threshold * prm->threshold * 0.9999f;
     p->border = prm->border;
@@ -440,7 +451,6 @@ static toed_status detect_chunk(toed_ctx* c, const toed_image* images, int n, co
     p->hyb = hyb ? 1 : 0;
     p->qad = prm->orientation == TOED_ORI_QAD ? 1 : 0;
     p->nms_to = nmsto ? 1 : 0;
-    p->det_rec = 1;
     p->ready = c->hb_ready;
     p->ready_epoch = c->hb_epoch;
     p->ready_spins = c->ready_spins;
@@ -456,7 +466,10 @@ static toed_status detect_chunk(toed_ctx* c, const toed_image* images, int n, co
     // for its size alone.)
     long long npx = 0, cum = 0;
     for (int i = 0; i < n; ++i) npx += (long long)images[i].width * images[i].height;
-    long long units = 0, tiles = 0, staging = 0;
+    long long units = 0, tiles = 0, staging = 0, segs = 0, ed = 0;
+    p->ed_rows = plan_ed_rows(images, n, c->num_sms);
+    for (int i = 0; i < n; ++i) segs += 2LL * images[i].height * ((images[i].width + kInner - 1) / kInner);
+    const int seg_tile = p->seg_tile = p->qad ? kSegTile : plan_seg_tile(segs);
     for (int i = 0; i < n; ++i) {
         const toed_image& im = images[i];
         DetImage& d = p->img[i];
@@ -478,29 +491,28 @@ static toed_status detect_chunk(toed_ctx* c, const toed_image* images, int n, co
         d.nsr = (im.height + d.S - 1) / d.S;
         d.unit_base = (int)units;
         d.tile_base = (int)tiles;
-        d.seg_base = tiles * kSegTile;
+        d.seg_base = tiles * seg_tile;
+        d.ed_base = (int)ed;
         d.wait_slot = wait_slot ? wait_slot[i] : 0;
-        d.tma_align = 1;
-        d.tma_boxw = 0;
-        if (async_rows)
-            d.tma = (d.dtype == TOED_F32) ? 2 : 0;  // async row copies (float32) or plain loads, never TMA
-        else if ((use && !use->staging) || plain_loads)
-            d.tma = 0;  // plain loads (host memory read in place: never TMA)
+        if (use && use->staging != 1)
+            d.tma = 0;  // loads prefetched in registers
         else
             encode_rows_map(&p->tmap[i], d, r);  // TMA where the image allows it (a host call per image)
         const long long nseg = 2LL * im.height * d.nsc;
         d.nseg = nseg;
         units += (long long)d.nsc * d.nsr;
-        tiles += (nseg + kSegTile - 1) / kSegTile;
+        tiles += (nseg + seg_tile - 1) / seg_tile;
+        ed += (long long)d.nsc * ((im.height + p->ed_rows - 1) / p->ed_rows);
         staging += im.capacity;
     }
-    if (units >= (1LL << 31) || tiles >= (1LL << 31)) return TOED_ERR_UNSUPPORTED;
+    if (units >= (1LL << 31) || tiles >= (1LL << 31) || ed >= (1LL << 31)) return TOED_ERR_UNSUPPORTED;
+    p->n_ed = (int)ed;
     p->n_units = (int)units;
     p->n_tiles = (int)tiles;
-    // every resident CTA may leave up to one reservation block of staging unused
+    // every resident warp may leave up to one reservation block of staging unused
     p->stage_blk = kStageBlk;
-    staging += resident * kStageBlk;
-    toed_status st = ensure_scratch(c, std::max(staging, 1LL), tiles * kSegTile, tiles, n, stream);
+    staging += resident * (kThreads / 32) * kStageBlk;
+    toed_status st = ensure_scratch(c, std::max(staging, 1LL), tiles * seg_tile, tiles, n, stream);
     if (st != TOED_OK) return st;
     p->sc.words = c->words;
     p->sc.staging = c->staging;
@@ -510,13 +522,10 @@ static toed_status detect_chunk(toed_ctx* c, const toed_image* images, int n, co
     p->sc.seg_cap = c->seg_cap;
     p->sc.tile_sum = c->tile_sum;
     p->sc.img_base = c->img_base;
-    // FP64 orientation recomputation: hybrid precision, grid orientation
-    // (the subpixel orientation replaces the staged one)
-    p->sc.refine = c->refine;
-    p->sc.refine_cap = (hyb && !p->qad) ? (int)std::min<long long>(c->refine_cap, 1LL << 30) : 0;
+    p->sc.seg_dst = c->seg_dst;
+    p->sc.tile_state = c->tile_state;
 
-    // the first chunk clears the flags and the refine-list length too; later
-    // chunks find the list emptied by the previous ordering pass
+    // the first chunk clears the flags too
     TOED_CU(cudaMemsetAsync(c->words, 0, (first_chunk ? kWords : 2) * sizeof(int), stream));
     const int grid = (int)std::min<long long>(units, resident);
     void* args[] = {p};
@@ -562,13 +571,12 @@ static toed_status check_batch(const toed_ctx* c, const toed_image* images, int 
 
 // The batch in chunks of kBatchMax images (caller holds c->mu, device set).
 static toed_status detect_all(toed_ctx* c, const toed_image* images, int n, const toed_params* prm,
-                              cudaStream_t stream, const toed_tuning* force = nullptr, bool plain_loads = false,
-                              const int* wait_slot = nullptr)
+                              cudaStream_t stream, const toed_tuning* force = nullptr, const int* wait_slot = nullptr)
 {
     const int r = radius_of(prm);
     toed_status st = TOED_OK;
     for (int i0 = 0; i0 < n && st == TOED_OK; i0 += kBatchMax)
-        st = detect_chunk(c, images + i0, std::min(kBatchMax, n - i0), prm, r, i0 == 0, stream, force, plain_loads,
+        st = detect_chunk(c, images + i0, std::min(kBatchMax, n - i0), prm, r, i0 == 0, stream, force,
                           wait_slot ? wait_slot + i0 : nullptr);
     return st;
 }
@@ -624,7 +632,7 @@ extern "C" toed_status toed_autotune(toed_ctx* c, const toed_image* images, int 
         // them (a small image's best height fills the resident CTAs once)
         static const int steps[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64};
         constexpr int kCand = (int)(sizeof(steps) / sizeof(steps[0]));
-        for (int staging = 2; staging >= 0 && st == TOED_OK; --staging)
+        for (int staging = 1; staging >= 0 && st == TOED_OK; --staging)  // (2 is 0's kernel path)
             for (int k = 0; k < kCand && st == TOED_OK; ++k) {
                 toed_tuning cand = {steps[k] * kStepRows - 2, staging, 0.f};
                 st = detect_all(c, images, n, prm, stream, &cand);  // untimed: scratch, caches
@@ -754,10 +762,11 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
             return fail(TOED_ERR_CUDA);                                                   \
         }                                                                                 \
     } while (0)
-    // Page-locked host outputs are written by the ordering pass itself
-    // (mapped into the device's address space; coherent over the C2C link):
-    // no count read-back and no list copies.  Otherwise lists go through
-    // device staging and are copied back per group once its counts are known.
+    // Page-locked host outputs are written by a kernel after the lists are
+    // complete, in whole lines through their mapping into the device's address
+    // space (coherent over the C2C link): no count read-back and no copy per
+    // list.  Otherwise lists are copied back per group once its counts are
+    // known.
     auto mapped = [](void* hp) -> void* {
         cudaPointerAttributes a;
         if (!hp || cudaPointerGetAttributes(&a, hp) != cudaSuccess) {
@@ -766,28 +775,21 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
         }
         return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
     };
-    // Page-locked inputs: with chunks == 1 the detection kernel reads them in
-    // place through their device mapping (zero copy over the C2C link); with
-    // more groups the copy engine brings the groups into device memory while
-    // ONE detection launch runs, each image's CTAs waiting (bounded) for its
-    // group's ready flag, which the copy engine writes after the group's
+    // Page-locked inputs: the copy engine brings the groups into device memory
+    // while ONE detection launch runs, each image's CTAs waiting (bounded) for
+    // its group's ready flag, which the copy engine writes after the group's
     // pixels -- every pixel crosses the link once and no group boundary
     // drains the GPU.  Pageable inputs: staged copies per group, one
     // detection launch per group once its copy is in.
     bool zin = true;
-    std::vector<const void*> in_map(n, nullptr);
-    for (int i = 0; i < n && zin; ++i) {
-        in_map[i] = mapped(const_cast<void*>(images[i].pixels));
-        zin = in_map[i] != nullptr;
-    }
+    for (int i = 0; i < n && zin; ++i) zin = mapped(const_cast<void*>(images[i].pixels)) != nullptr;
     // (flagged: one launch of at most kBatchMax images, so that nothing between
     // the launch and the copies' enqueueing can wait for the device; never
     // when launches run serialised -- CUDA_LAUNCH_BLOCKING, or a profiler or
     // checker injected into the runtime -- since then the waiting launch
     // would hold the host or the device until its wait gives up)
-    const bool inplace = zin && chunks == 1,
-               flagged = zin && chunks > 1 && n <= kBatchMax && !launches_serialised();
-    if (!inplace && (st = grow(&c->hb_in, &c->hb_in_cap, std::max(in_b, 1LL), stream)) != TOED_OK) return fail(st);
+    const bool flagged = zin && n <= kBatchMax && !launches_serialised();
+    if ((st = grow(&c->hb_in, &c->hb_in_cap, std::max(in_b, 1LL), stream)) != TOED_OK) return fail(st);
     if (flagged) {
         const long long had = c->hb_ready_cap;
         if ((st = grow(&c->hb_ready, &c->hb_ready_cap, (long long)chunks, stream)) != TOED_OK) return fail(st);
@@ -810,26 +812,21 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
     if (!c->s_in) TOED_HB(cudaStreamCreateWithFlags(&c->s_in, cudaStreamNonBlocking));
     if (!c->s_out) TOED_HB(cudaStreamCreateWithFlags(&c->s_out, cudaStreamNonBlocking));
     bool direct = true;
-    for (int i = 0; i < n && direct; ++i) {
-        void* e = mapped(images[i].edgels);
-        void* cn = mapped(images[i].count);
-        void* gi = images[i].grid_index ? mapped(images[i].grid_index) : nullptr;
-        direct = e && cn && (!images[i].grid_index || gi);
-        dev[i].edgels = e;
-        dev[i].count = static_cast<int*>(cn);
-        dev[i].grid_index = static_cast<int*>(gi);
-    }
+    std::vector<ListCopy> lists(n);
     for (int i = 0; i < n; ++i) {
-        dev[i].pixels = inplace ? in_map[i] : c->hb_in + in_off[i];
-        if (inplace) dev[i].pitch = images[i].pitch;
-        if (!direct) {
-            dev[i].edgels = c->hb_out + out_off[i];
-            dev[i].count = c->hb_cnt + i;
-            dev[i].grid_index = images[i].grid_index ? c->hb_idx + idx_off[i] : nullptr;
-        }
+        dev[i].pixels = c->hb_in + in_off[i];
+        dev[i].edgels = c->hb_out + out_off[i];
+        dev[i].count = c->hb_cnt + i;
+        dev[i].grid_index = images[i].grid_index ? c->hb_idx + idx_off[i] : nullptr;
+        ListCopy& l = lists[i];
+        l = {dev[i].edgels, mapped(images[i].edgels), dev[i].grid_index,
+             static_cast<int*>(images[i].grid_index ? mapped(images[i].grid_index) : nullptr), dev[i].count,
+             static_cast<int*>(mapped(images[i].count)), images[i].capacity};
+        direct = direct && l.dst && l.count_dst && (!l.idx || l.idx_dst);
     }
     for (int i = 0; i < n; ++i) {
         st = check_image(dev[i]);
+        if (st == TOED_OK && direct && (reinterpret_cast<uintptr_t>(lists[i].dst) & 15u) != 0) st = TOED_ERR_INVALID_ARG;
         if (st != TOED_OK) return fail(st);
     }
     // groups of consecutive images whose pixel counts grow geometrically
@@ -909,9 +906,11 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
         const int early = std::min(chunks, 2);
         for (int k = 0; k < early; ++k) TOED_HB(enqueue_group(k));
         TOED_HB(preload_finalize(radius_of(prm), prm->orientation == TOED_ORI_QAD));
-        st = detect_all(c, dev.data(), n, prm, stream, nullptr, true, slot.data());
+        TOED_HB(preload_list_copy());
+        st = detect_all(c, dev.data(), n, prm, stream, nullptr, slot.data());
         c->ready_spins = kReadySpinLimit;
         if (st != TOED_OK) return fail(st);
+        if (direct) TOED_HB(launch_list_copy(lists.data(), n, rec, stream));
         TOED_HB(cudaMemcpyAsync(c->hb_cnt + n, c->words + 2, sizeof(int), cudaMemcpyDeviceToDevice, stream));
         TOED_HB(cudaEventRecord(ev_det[0], stream));
         for (int k = early; k < chunks; ++k) TOED_HB(enqueue_group(k));
@@ -919,15 +918,16 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
         first[1] = n;
     } else {
         // 1. every group's images to the device, in order
-        for (int k = 0; k < chunks && !inplace; ++k) {
+        for (int k = 0; k < chunks; ++k) {
             TOED_HB(copy_group(k));
             TOED_HB(cudaEventRecord(ev_in[k], c->s_in));
         }
         // 2. detection of each group once its images are in
         for (int k = 0; k < chunks; ++k) {
-            if (!inplace) TOED_HB(cudaStreamWaitEvent(stream, ev_in[k], 0));
-            st = detect_all(c, dev.data() + first[k], first[k + 1] - first[k], prm, stream, nullptr, inplace);
+            TOED_HB(cudaStreamWaitEvent(stream, ev_in[k], 0));
+            st = detect_all(c, dev.data() + first[k], first[k + 1] - first[k], prm, stream);
             if (st != TOED_OK) return fail(st);
+            if (direct) TOED_HB(launch_list_copy(lists.data() + first[k], first[k + 1] - first[k], rec, stream));
             TOED_HB(cudaMemcpyAsync(c->hb_cnt + n + k, c->words + 2, sizeof(int), cudaMemcpyDeviceToDevice, stream));
             TOED_HB(cudaEventRecord(ev_det[k], stream));
         }

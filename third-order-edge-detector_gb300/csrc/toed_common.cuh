@@ -23,12 +23,12 @@ constexpr int kSizeClasses = 48;                   // launch size classes floor(
 constexpr int kThreads = 256;                      // threads per detection CTA
 constexpr int kExt = 32;                           // strip width incl. a 1-pixel ring each side
 constexpr int kInner = kExt - 2;                   // 30 output columns per strip
-constexpr int kHalves = kExt / 32;                 // warp-wide column groups of a strip
-constexpr int kRawRowBytes = 256;                  // bytes per staged input row (TMA box row) at most
 constexpr int kStepRows = 16;                      // original rows per sliding step (B)
 constexpr int kColRows = 8;                        // rows per column-pass thread (register blocking)
 constexpr int kSegTile = 1024;                     // segments per ordering-pass tile
-constexpr int kStageBlk = 256;                     // staging records a CTA reserves at a time
+constexpr int kEdRowsMax = 192;                    // image rows of an edgel-kernel tile at most
+constexpr int kScanTileMax = 4096;                 // segments per tile of a large launch's scan
+constexpr int kStageBlk = 64;                      // staging records a warp of the detection reserves at a time
 // Edgels whose third-order vector cancels by more than this factor (sum of
 // the terms' magnitudes over the largest component) get their orientation
 // recomputed from the image in FP64 (HYBRID precision, grid orientation).
@@ -57,7 +57,13 @@ __device__ __forceinline__ bool debug_in_bounds(bool ok, int* words, int line)
 #else
 #define TOED_IN_BOUNDS(cond, words) true
 #endif
-constexpr int kWords = 8;  // scratch words: [0] queue [1] cursor [2] flags [3] refine length [4] first bad line
+constexpr int kWords = 8;  // scratch words: [0] queue [1] cursor [2] flags [3] tile ticket [4] first bad line
+
+// Floats of a staged input row of the detection (a multiple of 16 bytes): the
+// window of kExt outputs at radius r, up to three floats of alignment before
+// it and one past an odd window's last pair.
+// An odd number of 16-byte groups: eight rows apart before a column meets its bank again.
+constexpr int staged_width(int r) { return ((kExt + 2 * r + 2 + 4 + (r & 1) + 3) / 4 | 1) * 4; }
 
 // 1-D taps, index k <-> offset x = k - (r+1) (+0.5 for the shifted set).
 // Filters: 0 G, 1 Gx, 2 Gxx, 3 Gxxx, 4..7 the same shifted by +0.5.
@@ -87,51 +93,62 @@ struct DetImage {
     int S;               // strip inner rows of this image's work units (multiple of kStepRows minus 2)
     int unit_base;       // first work unit
     int tile_base;       // first ordering tile
-    int tma;             // 1: rows arrive by TMA through BatchParams::tmap[k]; 2: by per-thread async
-                         // copies (float32, any address); 0: plain loads
-    int tma_align;       // element alignment of a TMA box's x coordinate (16 bytes)
-    int tma_boxw;        // box width in elements (the halo row plus the alignment shift)
+    int ed_base;         // first edgel-kernel tile
+    int tma;             // 1: rows arrive by TMA through BatchParams::tmap[k]; 0: by loads
     int wait_slot;       // 0: pixels ready at launch; g > 0: the copy engine is still bringing them in,
                          // BatchParams::ready[g - 1] reads ready_epoch once they are complete
 };
 
 struct Scratch {
-    int* words;          // kWords: [0] unit queue, [1] staging cursor, [2] flags, [3] refine-list length,
-                         // [4] (bounds-checked builds) source line of the first failed check
-    double4_32a* staging;  // staged edgels: TO correction (x, y, orientation, strength); the
-                           // detection uses the same memory as float4 records (det_stage)
+    int* words;          // kWords: [0] unit queue, [1] staging cursor, [2] flags, [3] the scan's tile
+                         // ticket, [4] (bounds-checked builds) source line of the first failed check
+    double4_32a* staging;  // staged edgels, 32 bytes each: TO correction (x, y, orientation, strength);
+                           // the detection two float4 (det_stage)
     int* staging_idx;
     long long staging_cap;
     int2* seg;           // per segment {staging offset, count}
     long long seg_cap;   // segments `seg` holds
     int* tile_sum;       // per ordering tile
     long long* img_base; // per image: exclusive prefix of its first segment
-    int4* refine;        // edgels whose orientation is recomputed in FP64: {staging slot, image, Gr, Gc}
-    int refine_cap;      // entries of `refine` (0: no recomputation)
+    int* seg_dst;        // per segment: its place in its image's list
+    unsigned long long* tile_state;  // per scan tile: {0, 1 its count, 2 the count of its image's
+                                     // tiles up to it} << 32 | count
 };
 
-// The detection's staged edgel: a float4 in the staging memory beside the
-// 2x-grid index in staging_idx (20 bytes per edgel).  x, y hold what the
-// output's FP64 position is rebuilt from without loss: in HYBRID precision
-// the subpixel offset 0.5 s* n (the grid part 0.5 (G - 1) is exact), in
-// FP32 precision the FP32 position G + s* n on the 2x grid; then the
-// orientation and the strength.
+// The detection's staged edgel, two float4: (Ix, Iy, |grad I| at the axis and
+// the diagonal neighbour ahead), (the same behind, the 2x-grid index's bits,
+// unused).
 __device__ __forceinline__ float4* det_stage(const Scratch& sc) { return reinterpret_cast<float4*>(sc.staging); }
 
-// Output position (x, y) = ((pos - 1) / 2) of a staged edgel (cpu_toed.cpp:516-521).
-__device__ __forceinline__ double2 det_xy(const float4& rec, int idx, int W2, bool hyb)
+__device__ __forceinline__ float sqrt_approx(float x)
 {
-    const int Gr = idx / W2, Gc = idx - Gr * W2;
-    if (hyb)
-        return make_double2((double)(0.5f * (float)(Gc - 1)) + (double)rec.x,
-                            (double)(0.5f * (float)(Gr - 1)) + (double)rec.y);
-    return make_double2(((double)rec.x - 1.0) * 0.5, ((double)rec.y - 1.0) * 0.5);
+    float y;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// |grad I| at a 2x-grid point from its (Ix, Iy); the NMS decision and the
+// peak fit both use this one expression.
+__device__ __forceinline__ float grad_mag(float2 g) { return sqrt_approx(fmaf(g.x, g.x, g.y * g.y)); }
+
+// The third-order vector (cpu_toed.cpp:227-230) in FP32 with its shared
+// products factored out, d = fxx, fxy, fyy, fxxy, fxyy, fxxx, fyyy:
+// TIx = 2 (fx (fxx^2 + fxy^2) + fy fxy (fxx + fyy) + fx fy fxxy) + fy^2 fxyy + fx^2 fxxx
+// TIy = 2 (fx fxy (fxx + fyy) + fy (fyy^2 + fxy^2) + fx fy fxyy) + fx^2 fxxy + fy^2 fyyy
+__device__ __forceinline__ void to_vec32(float gx, float gy, const float (&d)[7], float* tix, float* tiy)
+{
+    const float fxx = d[0], fxy = d[1], fyy = d[2], fxxy = d[3], fxyy = d[4], fxxx = d[5], fyyy = d[6];
+    const float a2 = fmaf(fxx, fxx, fxy * fxy), c2 = fmaf(fyy, fyy, fxy * fxy), bc = fxy * (fxx + fyy);
+    const float pxy = gx * gy, x2 = gx * gx, y2 = gy * gy;
+    *tix = fmaf(2.f, fmaf(gx, a2, fmaf(gy, bc, pxy * fxxy)), fmaf(y2, fxyy, x2 * fxxx));
+    *tiy = fmaf(2.f, fmaf(gx, bc, fmaf(gy, c2, pxy * fxyy)), fmaf(x2, fxxy, y2 * fyyy));
 }
 
 struct BatchParams {
-    CUtensorMap tmap[kBatchMax];  // per image: 2-D map, box (tma_boxw x kStepRows), OOB zero fill
+    CUtensorMap tmap[kBatchMax];  // per image: 2-D map, box (staged_width x kStepRows), OOB zero fill
     TapBlock taps;
     TapBlock64 taps64;
+    float2 ytap[2][kMaxTaps];  // (Gy, G) of the whole and the half-pixel shifted set: the column pass's pairs
     float thr;
     float thr2;          // candidate prefilter on |grad I|^2: a little below thr^2 (-1 when thr < 0)
     int border;
@@ -142,13 +159,14 @@ struct BatchParams {
     int n_tiles;
     int out_f64;
     int radius;
-    int stage_blk;       // staging records reserved per atomic (1: exactly each step's edgels)
+    int stage_blk;       // staging records a warp reserves per atomic (1: exactly each step's edgels)
+    int seg_tile;        // segments per ordering tile: kSegTile, or kScanTileMax
+    int ed_rows;         // image rows of an edgel-kernel tile (one strip column wide), up to kEdRowsMax
+    int n_ed;            // such tiles
     int hyb;             // 1: peak fit on exact FP32 differences, FP64 recomputation of ill-conditioned
                          // orientations (TOED_HYBRID)
     int qad;             // 1: orientation from derivatives interpolated at the subpixel point (TOED_ORI_QAD)
     int nms_to;          // 1: NMS and peak fit along the corrected normal (TOED_NMS_TO_NORMAL)
-    int det_rec;         // ordering pass input: 1 the detection's float4 records (det_stage), 0 the TO
-                         // correction's double4 records
     const int* ready;    // per copy group: ready_epoch once the group's images are in device memory
     int ready_epoch;
     int ready_spins;     // polls of a ready flag before the wait gives up (TOED_FLAG_TIMEOUT)
@@ -189,6 +207,78 @@ __device__ __forceinline__ int block_excl_scan(int v, int* s_warp, int* total)
     __syncthreads();
     return r;
 }
+
+// ---------------------------------------------------------------------------
+// TMA staging of input rows (cp.async.bulk.tensor + mbarrier)
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t smem_addr(const void* p)
+{
+    return (uint32_t)__cvta_generic_to_shared(p);
+}
+
+__device__ __forceinline__ void mbar_init(uint32_t bar)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+
+// One thread: one box of kStepRows rows at (x, y) of image map `tm` into `dst`.
+__device__ __forceinline__ void tma_copy_rows(const CUtensorMap* tm, uint32_t dst, uint32_t bar, int x, int y)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            dst),
+        "l"(reinterpret_cast<uint64_t>(tm)), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_rows(const CUtensorMap* tm, uint32_t dst, uint32_t bar, int x, int y,
+                                              uint32_t bytes)
+{
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    tma_copy_rows(tm, dst, bar, x, y);
+}
+
+// Bounded wait for the mbarrier phase: gives up after ~2^20 polls (each poll
+// may suspend briefly) instead of hanging the SM.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase)
+{
+    for (int i = 0; i < (1 << 20); ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+            : "=r"(ok)
+            : "r"(bar), "r"(phase)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
+// Programmatic dependent launch: a kernel launched so (launch_after) may start
+// while its predecessor in the stream still runs, once all of that one's CTAs
+// have called launch_dependents() or ended; what it reads of the predecessors'
+// results it reads after grid_wait(), which returns when they are complete.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+inline cudaError_t launch_after(const void* func, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t stream)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, func, args);
+}
+
+// x rounded down to a multiple of 4 (floats: 16 bytes, where a TMA box may start).
+__device__ __forceinline__ int floor4(int x) { return x >= 0 ? x & ~3 : -((3 - x) & ~3); }
 
 // Index of the image whose [base, next base) range holds `u` (bases ascending).
 template <typename GetBase>

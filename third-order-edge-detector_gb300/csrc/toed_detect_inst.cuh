@@ -6,19 +6,9 @@
 
 #define TOED_DETECT_INSTANCE(R)                                                    \
     namespace toed {                                                               \
-    DetectEntry detect_entry_r##R(bool hyb, bool async, bool nmsto)                \
+    DetectEntry detect_entry_r##R(bool nmsto)                                      \
     {                                                                              \
-        DetectEntry e;                                                             \
-        e.smem = Cfg<R>::smem;                                                     \
-        if (nmsto)                                                                 \
-            e.func = hyb ? (const void*)toed_detect_kernel<R, true, false, true>   \
-                         : (const void*)toed_detect_kernel<R, false, false, true>; \
-        else if (async)                                                            \
-            e.func = hyb ? (const void*)toed_detect_kernel<R, true, true>          \
-                         : (const void*)toed_detect_kernel<R, false, true>;        \
-        else                                                                       \
-            e.func = hyb ? (const void*)toed_detect_kernel<R, true, false>         \
-                         : (const void*)toed_detect_kernel<R, false, false>;       \
-        return e;                                                                  \
+        if (nmsto) return {(const void*)toed_detect_kernel<R, true>, Cfg<R, true>::smem}; \
+        return {(const void*)toed_detect_kernel<R>, Cfg<R>::smem};                 \
     }                                                                              \
     }

@@ -1,92 +1,24 @@
-// toed_finalize.cu -- ordering pass: turns the detection kernel's staged
-// edgels and row-segment table into each image's edgel list in the
-// reference's order (row-major over the 2x grid, cpu_toed.cpp:510-538).
+// toed_finalize.cu -- ordering pass of the TO correction and of the
+// quick-and-dirty orientation mode: turns staged edgels and the row-segment
+// table into each image's edgel list in the reference's order (row-major,
+// cpu_toed.cpp:510-538).  (The detection's other modes are ordered by the
+// edgel kernel itself, toed_edgels.cu.)
 //
-// Segments are (2x-grid row, strip column) pairs laid out row-major per image
-// and padded to whole tiles of kSegTile.  Three short kernels:
-//   fin_tile_sums : edgels per tile; then the FP64 orientation recomputation
-//                   of the edgels the detection kernel listed
+// Segments are (row, strip column) pairs laid out row-major per image and
+// padded to whole tiles of kSegTile.  Three short kernels:
+//   fin_tile_sums : edgels per tile
 //   fin_tile_scan : exclusive scan over tiles; per-image base and count,
 //                   capacity flag
 //   fin_scatter   : per tile, scan the segment counts, then copy the tile's
 //                   staged records cooperatively to their list positions
 //                   (global prefix - image base), converting to the output
-//                   dtype.
+//                   dtype (the quick-and-dirty mode: toed_qad.cu).
+#include <algorithm>
+
 #include "toed_common.cuh"
 #include "toed_internal.h"
 
 namespace toed {
-
-// One listed edgel, one warp: the nine derivatives at 2x-grid point
-// (Gr, Gc) = (2i + a, 2j + b) straight from the image with FP64 taps, zero
-// outside the image -- the (2r+1)^2 window of unshifted taps on sub-grid
-// (0, 0) (cpu_toed.cpp:205-221), the (2r+3)^2 window with the half-pixel
-// shifted taps along the odd axes elsewhere (cpu_toed.cpp:246-344) -- then the
-// third-order vector (cpu_toed.cpp:227-232) and its angle in FP64, written
-// over the staged orientation.  Lane t forms the four column-filtered sums of
-// window row t; the row filters then weight them and the warp reduces.
-constexpr int kRefineChunk = 9;
-
-__device__ void refine_edgel(const BatchParams& p, int4 e, int lane)
-{
-    const DetImage& im = p.img[e.y];
-    const int r = p.radius;
-    const int i = e.z >> 1, a = e.z & 1, j = e.w >> 1, b = e.w & 1;
-    const int h = (a | b) ? r + 1 : r;
-    const double* X = &p.taps64.v[b ? 4 : 0][0];  // filter f, tap k: X[f * kMaxTaps + k]
-    const double* Y = &p.taps64.v[a ? 4 : 0][0];
-    const int dp = lane - h, row = i - dp;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0, y0 = 0.0, y1 = 0.0, y2 = 0.0, y3 = 0.0;
-    if (lane <= 2 * h && row >= 0 && row < im.H) {
-        // the row in chunks of kRefineChunk columns, each chunk's loads
-        // first (independent, so in flight together)
-        const long long ro = (long long)row * im.pitch;
-        const bool u8 = im.dtype == TOED_U8;
-        const int k0 = r + 1 - h;  // tap of column offset q = -h
-        for (int c0 = 0; c0 <= 2 * h; c0 += kRefineChunk) {
-            float v[kRefineChunk];
-#pragma unroll
-            for (int t = 0; t < kRefineChunk; ++t) {
-                const int col = j + h - (c0 + t);  // column offset q = c0 + t - h
-                v[t] = 0.f;
-                if (c0 + t <= 2 * h && col >= 0 && col < im.W)
-                    v[t] = u8 ? (float)static_cast<const unsigned char*>(im.src)[ro + col]
-                              : static_cast<const float*>(im.src)[ro + col];
-            }
-#pragma unroll
-            for (int t = 0; t < kRefineChunk; ++t) {
-                if (c0 + t > 2 * h) break;
-                const double x = v[t];
-                const int kq = k0 + c0 + t;
-                s0 = fma(x, X[kq], s0);
-                s1 = fma(x, X[kMaxTaps + kq], s1);
-                s2 = fma(x, X[2 * kMaxTaps + kq], s2);
-                s3 = fma(x, X[3 * kMaxTaps + kq], s3);
-            }
-        }
-        const int kp = dp + r + 1;
-        y0 = Y[kp];
-        y1 = Y[kMaxTaps + kp];
-        y2 = Y[2 * kMaxTaps + kp];
-        y3 = Y[3 * kMaxTaps + kp];
-    }
-    // fx fy fxx fxy fyy fxxy fxyy fxxx fyyy
-    double d[9] = {y0 * s1, y1 * s0, y0 * s2, y1 * s1, y2 * s0, y1 * s2, y2 * s1, y0 * s3, y3 * s0};
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int f = 0; f < 9; ++f) d[f] += __shfl_xor_sync(0xffffffffu, d[f], o);
-    if (lane == 0) {
-        const double fx = d[0], fy = d[1], fxx = d[2], fxy = d[3], fyy = d[4], fxxy = d[5], fxyy = d[6],
-                     fxxx = d[7], fyyy = d[8];
-        const double tix = fx * (2 * fxx * fxx + 2 * fxy * fxy) + fy * (2 * fxx * fxy + 2 * fyy * fxy) +
-                           2 * fx * fy * fxxy + fy * fy * fxyy + fx * fx * fxxx;
-        const double tiy = fx * (2 * fxx * fxy + 2 * fyy * fxy) + fy * (2 * fyy * fyy + 2 * fxy * fxy) +
-                           2 * fx * fy * fxyy + fx * fx * fxxy + fy * fy * fyyy;
-        const double ori = (tix == 0.0 && tiy == 0.0) ? __longlong_as_double(0x7ff8000000000000LL) : atan2(tix, -tiy);
-        det_stage(p.sc)[e.x].z = (float)ori;
-    }
-}
 
 __global__ void __launch_bounds__(256) fin_tile_sums(const __grid_constant__ BatchParams p)
 {
@@ -104,13 +36,6 @@ __global__ void __launch_bounds__(256) fin_tile_sums(const __grid_constant__ Bat
     int total;
     block_excl_scan<256>(sum, s_warp, &total);
     if (threadIdx.x == 0) p.sc.tile_sum[t] = total;
-    if (p.sc.refine_cap > 0) {
-        const int nref = min(p.sc.words[3], p.sc.refine_cap);
-        // entry q to warp q / gridDim of block q % gridDim: a short list
-        // spreads over all SMs' FP64 pipes
-        const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-        for (int q = w; q < nref; q += gridDim.x * 8) refine_edgel(p, p.sc.refine[q], lane);
-    }
 }
 
 __global__ void __launch_bounds__(1024) fin_tile_scan(const __grid_constant__ BatchParams p)
@@ -134,7 +59,6 @@ __global__ void __launch_bounds__(1024) fin_tile_scan(const __grid_constant__ Ba
         *p.img[k].count = cnt;
         if (cnt > p.img[k].cap) atomicOr(&p.sc.words[2], TOED_FLAG_OVER_CAPACITY);
     }
-    if (threadIdx.x == 0) p.sc.words[3] = 0;  // refine list empty for the next launch (fin_tile_sums has read it)
 }
 
 // One CTA per tile of kSegTile segments: an exclusive scan gives every
@@ -181,17 +105,7 @@ __global__ void __launch_bounds__(kFinThreads) fin_scatter(const __grid_constant
         }
         const long long d = base + r, src = (long long)s_src[lo] + (r - s_dst[lo]);
         if (d >= cap || src >= p.sc.staging_cap) continue;
-        double4_32a rc;
-        int gi = 0;
-        if (p.det_rec) {  // the detection's compact record
-            const float4 st = det_stage(p.sc)[src];
-            gi = p.sc.staging_idx[src];
-            const double2 xy = det_xy(st, gi, 2 * im.W, p.hyb != 0);
-            rc = make_double4_32a(xy.x, xy.y, (double)st.z, (double)st.w);
-        } else {
-            rc = p.sc.staging[src];
-            if (im.index) gi = p.sc.staging_idx[src];
-        }
+        const double4_32a rc = p.sc.staging[src];
         if (p.out_f64) {  // two 16-byte stores: the caller's buffer need only be 16-byte aligned
             double2* o = reinterpret_cast<double2*>(im.out) + 2 * d;
             o[0] = make_double2(rc.x, rc.y);
@@ -199,27 +113,83 @@ __global__ void __launch_bounds__(kFinThreads) fin_scatter(const __grid_constant
         } else {
             reinterpret_cast<float4*>(im.out)[d] = make_float4((float)rc.x, (float)rc.y, (float)rc.z, (float)rc.w);
         }
-        if (im.index) im.index[d] = gi;
     }
+}
+
+// Lists to mapped host memory: whole lines written by consecutive threads.
+// (The edgel kernel's own stores are single records at scattered places: over
+// the link they took 0.45 ms more per 40 MB of lists.)
+struct ListCopies {
+    ListCopy l[kBatchMax];
+    int rec;
+};
+
+__global__ void __launch_bounds__(256) fin_list_copy(const __grid_constant__ ListCopies p)
+{
+    const ListCopy& l = p.l[blockIdx.y];
+    const int cnt = *l.count, n = min(cnt, l.cap);
+    const long long nv = (long long)n * p.rec / 16;
+    const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, st = (long long)gridDim.x * blockDim.x;
+    const uint4* src = static_cast<const uint4*>(l.src);
+    uint4* dst = static_cast<uint4*>(l.dst);
+    for (long long i = t0; i < nv; i += st) dst[i] = src[i];
+    if (l.idx)
+        for (long long i = t0; i < n; i += st) l.idx_dst[i] = l.idx[i];
+    if (t0 == 0) *l.count_dst = cnt;
+}
+
+cudaError_t preload_list_copy()
+{
+    cudaFuncAttributes fa;
+    return cudaFuncGetAttributes(&fa, (const void*)fin_list_copy);
+}
+
+cudaError_t launch_list_copy(const ListCopy* lists, int n, int rec, cudaStream_t stream)
+{
+    for (int i0 = 0; i0 < n; i0 += kBatchMax) {
+        ListCopies p;
+        const int m = n - i0 < kBatchMax ? n - i0 : kBatchMax;
+        for (int i = 0; i < m; ++i) p.l[i] = lists[i0 + i];
+        p.rec = rec;
+        void* args[] = {&p};
+        // enough stores in flight to fill the link whatever the number of lists
+        const cudaError_t e = cudaLaunchKernel((const void*)fin_list_copy, dim3(std::max(8, 1024 / m), m), dim3(256), args, 0, stream);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t preload_finalize(int radius, bool qad)
 {
+    if (!qad) return preload_edgels(radius);
     cudaFuncAttributes fa;
     cudaError_t e = cudaFuncGetAttributes(&fa, (const void*)fin_tile_sums);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)fin_tile_scan);
-    if (e == cudaSuccess) e = qad ? preload_scatter_qad(radius) : cudaFuncGetAttributes(&fa, (const void*)fin_scatter);
+    if (e == cudaSuccess) e = preload_scatter_qad(radius);
+    return e;
+}
+
+// Tile sums and their scan over the whole launch.
+static cudaError_t launch_tile_scan(const BatchParams& p, cudaStream_t stream)
+{
+    void* args[] = {const_cast<BatchParams*>(&p)};
+    cudaError_t e = cudaLaunchKernel((const void*)fin_tile_sums, dim3(p.n_tiles), dim3(256), args, 0, stream);
+    if (e == cudaSuccess) e = cudaLaunchKernel((const void*)fin_tile_scan, dim3(1), dim3(1024), args, 0, stream);
     return e;
 }
 
 cudaError_t launch_finalize(const BatchParams& p, cudaStream_t stream)
 {
+    if (!p.qad) return launch_edgels(p, stream);
+    const cudaError_t e = launch_tile_scan(p, stream);
+    return e == cudaSuccess ? launch_scatter_qad(p, stream) : e;
+}
+
+cudaError_t launch_finalize_subpix(const BatchParams& p, cudaStream_t stream)
+{
+    const cudaError_t e = launch_tile_scan(p, stream);
+    if (e != cudaSuccess) return e;
     void* args[] = {const_cast<BatchParams*>(&p)};
-    cudaError_t e = cudaLaunchKernel((const void*)fin_tile_sums, dim3(p.n_tiles), dim3(256), args, 0, stream);
-    if (e != cudaSuccess) return e;
-    e = cudaLaunchKernel((const void*)fin_tile_scan, dim3(1), dim3(1024), args, 0, stream);
-    if (e != cudaSuccess) return e;
-    if (p.qad) return launch_scatter_qad(p, stream);
     return cudaLaunchKernel((const void*)fin_scatter, dim3(p.n_tiles), dim3(kFinThreads), args, 0, stream);
 }
 

@@ -14,13 +14,32 @@ struct DetectEntry {
     size_t smem;
 };
 
-// Per-radius instantiations (toed_detect_r<R>.cu); hyb selects the FP64
-// epilogue, async the variant that stages rows by per-thread async copies,
-// nmsto the corrected-normal NMS (rows by TMA or plain loads).
-DetectEntry detect_entry(int radius, bool hyb, bool async = false, bool nmsto = false);
+// Per-radius instantiations (toed_detect_r<R>.cu); nmsto: the corrected-normal NMS.
+DetectEntry detect_entry(int radius, bool nmsto = false);
 
+// What follows the detection kernel (toed_edgels.cu, toed_qad.cu) and the TO
+// correction's kernels: the edgel lists.
 cudaError_t launch_finalize(const BatchParams& p, cudaStream_t stream);
-// Load the ordering pass' kernels for `radius` (and the QaD variant) now:
+cudaError_t launch_finalize_subpix(const BatchParams& p, cudaStream_t stream);
+cudaError_t launch_edgels(const BatchParams& p, cudaStream_t stream);
+cudaError_t preload_edgels(int radius);
+cudaError_t prepare_edgels(int radius);  // its attributes, once per device and radius
+
+// One finished list from device memory to its mapped host buffers
+// (toed_finalize.cu): min(count, cap) records of `rec` bytes, the grid
+// indices where wanted, and the count.
+struct ListCopy {
+    const void* src;
+    void* dst;
+    const int* idx;
+    int* idx_dst;
+    const int* count;
+    int* count_dst;
+    int cap;
+};
+cudaError_t launch_list_copy(const ListCopy* lists, int n, int rec, cudaStream_t stream);
+cudaError_t preload_list_copy();
+// Load those kernels for `radius` (and the QaD variant) now:
 // with lazy module loading a kernel's first launch may wait for the device,
 // which must not happen while a detection launch waits for copies that the
 // host has yet to enqueue.
@@ -29,15 +48,20 @@ cudaError_t preload_finalize(int radius, bool qad);
 cudaError_t launch_scatter_qad(const BatchParams& p, cudaStream_t stream);
 cudaError_t preload_scatter_qad(int radius);
 
+// The taps of (sigma, r) in FP64, and each rounded once to FP32; BatchParams::ytap from the latter.
+void make_taps64(double sigma, int r, TapBlock64* tb);
+void make_taps(double sigma, int r, TapBlock* tb);
+void make_ytap(const TapBlock& t, float2 (*ytap)[kMaxTaps]);
+
 // Host-side checks of one device image (pointers, sizes, dtype, the
 // 16-byte edgel and 4-byte float32 pixel alignment): TOED_OK or the status
 // every detection entry point returns for it.
 toed_status check_image(const toed_image& im);
 
-// Fill d.tma / d.tma_align / d.tma_boxw and encode the image's row map for
-// TMA staging (kStepRows-row boxes, zero fill outside the image).  Leaves
-// d.tma = 0 -- plain loads -- when the driver entry point is unavailable or
-// the image's base or pitch is not 16-byte aligned.
+// Fill d.tma and encode the image's row map for TMA staging (kStepRows-row
+// boxes, zero fill outside the image).  Leaves d.tma = 0 -- loads -- for 8-bit
+// pixels, which have to be converted anyway, and when the driver entry point
+// is unavailable or the image's base or pitch is not 16-byte aligned.
 void encode_rows_map(CUtensorMap* m, DetImage& d, int radius);
 
 // Enqueue the adjoint (toed_backward.cu): clears each item's grad_pixels,

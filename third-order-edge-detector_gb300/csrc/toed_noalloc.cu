@@ -40,9 +40,6 @@
 #include "toed_internal.h"
 
 namespace toed {
-void make_taps(double sigma, int r, TapBlock* tb);
-void make_taps64(double sigma, int r, TapBlock64* tb);
-
 namespace {
 
 constexpr long long kNaMaxPixels = TOED_NOALLOC_MAX_PIXELS;
@@ -51,17 +48,17 @@ constexpr long long kNaMaxEdgels = TOED_NOALLOC_MAX_EDGELS;
 // segments 2H x ceil(W/30) <= pixels/15 + 2H, padded to whole ordering tiles
 constexpr long long kNaMaxTiles = (kNaMaxPixels / 15 + 2LL * kNaMaxDim) / kSegTile + 2;
 constexpr long long kNaMaxSegs = kNaMaxTiles * kSegTile;
-constexpr long long kNaRefine = kNaMaxEdgels / 64 + 1024;  // orientation recomputation list
 
 constexpr size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 constexpr size_t kOffWords = 0;
 constexpr size_t kOffStaging = align256(kOffWords + kWords * sizeof(int));
 constexpr size_t kOffIdx = align256(kOffStaging + sizeof(double4_32a) * kNaMaxEdgels);
 constexpr size_t kOffSeg = align256(kOffIdx + sizeof(int) * kNaMaxEdgels);
-constexpr size_t kOffTiles = align256(kOffSeg + sizeof(int2) * kNaMaxSegs);
+constexpr size_t kOffDst = align256(kOffSeg + sizeof(int2) * kNaMaxSegs);
+constexpr size_t kOffTiles = align256(kOffDst + sizeof(int) * kNaMaxSegs);
 constexpr size_t kOffBase = align256(kOffTiles + sizeof(int) * kNaMaxTiles);
-constexpr size_t kOffRefine = align256(kOffBase + sizeof(long long));
-constexpr size_t kScratchBytes = align256(kOffRefine + sizeof(int4) * kNaRefine);
+constexpr size_t kOffState = align256(kOffBase + sizeof(long long));
+constexpr size_t kScratchBytes = align256(kOffState + sizeof(unsigned long long) * kNaMaxTiles);
 
 // The fixed scratch (see the file comment): about 11 MB per device.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
@@ -70,13 +67,12 @@ constexpr int kMaxDevices = 64;
 std::mutex g_mu;
 unsigned char* g_dev_scratch[kMaxDevices] = {};
 int g_dev_sms[kMaxDevices] = {};
-int g_dev_bps[kMaxDevices][TOED_MAX_RADIUS + 1][2][2] = {};  // resident CTAs per SM [radius][hybrid][TO normal]
+int g_dev_bps[kMaxDevices][TOED_MAX_RADIUS + 1][2] = {};  // resident CTAs per SM [radius][TO normal]
 
 // Device address of g_noalloc_scratch on `dev` (current), the device's SM
 // count and the detection kernel's occupancy, looked up once per device
-// (and radius / precision) so that later calls make no such queries.
-cudaError_t device_setup(int dev, int r, bool hyb, bool nmsto, const DetectEntry& ent, unsigned char** base, int* sms,
-                         int* bps)
+// (and radius) so that later calls make no such queries.
+cudaError_t device_setup(int dev, int r, bool nmsto, const DetectEntry& ent, unsigned char** base, int* sms, int* bps)
 {
     std::lock_guard<std::mutex> lk(g_mu);
     if (!g_dev_scratch[dev]) {
@@ -89,7 +85,7 @@ cudaError_t device_setup(int dev, int r, bool hyb, bool nmsto, const DetectEntry
         g_dev_sms[dev] = n;
         g_dev_scratch[dev] = static_cast<unsigned char*>(ptr);
     }
-    int& b = g_dev_bps[dev][r][hyb ? 1 : 0][nmsto ? 1 : 0];
+    int& b = g_dev_bps[dev][r][nmsto ? 1 : 0];
     if (b == 0) {
         cudaError_t e = cudaFuncSetAttribute(ent.func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ent.smem);
         if (e != cudaSuccess) return e;
@@ -97,6 +93,8 @@ cudaError_t device_setup(int dev, int r, bool hyb, bool nmsto, const DetectEntry
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ent.func, kThreads, ent.smem);
         if (e != cudaSuccess) return e;
         if (n <= 0) return cudaErrorInvalidConfiguration;
+        e = prepare_edgels(r);
+        if (e != cudaSuccess) return e;
         b = n;
     }
     *base = g_dev_scratch[dev];
@@ -131,19 +129,20 @@ extern "C" toed_status toed_detect_noalloc(const toed_image* im, const toed_para
     const int r = prm->radius > 0 ? prm->radius : (int)std::ceil(4.0 * (double)prm->sigma);
     if (r < 1 || r > TOED_MAX_RADIUS) return TOED_ERR_UNSUPPORTED;
     const bool nmsto = prm->nms_direction == TOED_NMS_TO_NORMAL;
-    const DetectEntry ent = detect_entry(r, prm->precision != TOED_FP32, false, nmsto);
+    const DetectEntry ent = detect_entry(r, nmsto);
     if (!ent.func) return TOED_ERR_UNSUPPORTED;
 
     int dev = 0, sms = 0, bps = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return TOED_ERR_CUDA;
     unsigned char* base = nullptr;
-    if (device_setup(dev, r, prm->precision != TOED_FP32, nmsto, ent, &base, &sms, &bps) != cudaSuccess)
+    if (device_setup(dev, r, nmsto, ent, &base, &sms, &bps) != cudaSuccess)
         return TOED_ERR_CUDA;
 
     BatchParams p;  // on the stack: no heap allocation either
     std::memset(&p, 0, sizeof(p));
-    make_taps((double)prm->sigma, r, &p.taps);
     make_taps64((double)prm->sigma, r, &p.taps64);
+    make_taps((double)prm->sigma, r, &p.taps);
+    make_ytap(p.taps, p.ytap);
     p.thr = prm->threshold;
     p.thr2 = prm->threshold < 0.f ? -1.f : prm->threshold * prm->threshold * 0.9999f;
     p.border = prm->border;
@@ -153,7 +152,6 @@ extern "C" toed_status toed_detect_noalloc(const toed_image* im, const toed_para
     p.hyb = prm->precision != TOED_FP32 ? 1 : 0;
     p.qad = prm->orientation == TOED_ORI_QAD ? 1 : 0;
     p.nms_to = nmsto ? 1 : 0;
-    p.det_rec = 1;
     p.stage_blk = 1;  // staging sized to the capacity exactly: reserve each step's edgels alone
     // strip height: the tallest of 254 / 126 / 62 / 30 / 14 rows that still
     // gives every resident CTA a few strips
@@ -183,10 +181,14 @@ extern "C" toed_status toed_detect_noalloc(const toed_image* im, const toed_para
     d.nsr = (im->height + S - 1) / S;
     d.unit_base = 0;
     d.tile_base = 0;
+    d.ed_base = 0;
+    p.ed_rows = 64;
+    p.n_ed = nsc * ((im->height + p.ed_rows - 1) / p.ed_rows);
     d.seg_base = 0;
     d.nseg = 2LL * im->height * nsc;
     encode_rows_map(&p.tmap[0], d, r);
     p.n_units = d.nsc * d.nsr;
+    p.seg_tile = kSegTile;
     p.n_tiles = (int)((d.nseg + kSegTile - 1) / kSegTile);
     p.sc.words = reinterpret_cast<int*>(base + kOffWords);
     p.sc.staging = reinterpret_cast<double4_32a*>(base + kOffStaging);
@@ -196,10 +198,10 @@ extern "C" toed_status toed_detect_noalloc(const toed_image* im, const toed_para
     p.sc.seg_cap = kNaMaxSegs;
     p.sc.tile_sum = reinterpret_cast<int*>(base + kOffTiles);
     p.sc.img_base = reinterpret_cast<long long*>(base + kOffBase);
-    p.sc.refine = reinterpret_cast<int4*>(base + kOffRefine);
-    p.sc.refine_cap = (p.hyb && !p.qad) ? (int)kNaRefine : 0;
+    p.sc.seg_dst = reinterpret_cast<int*>(base + kOffDst);
+    p.sc.tile_state = reinterpret_cast<unsigned long long*>(base + kOffState);
 
-    // queue, staging cursor, flags and refine-list length start at zero on every call
+    // queue, staging cursor and flags start at zero on every call
     if (cudaMemsetAsync(p.sc.words, 0, kWords * sizeof(int), stream) != cudaSuccess) return TOED_ERR_CUDA;
     const int grid = (int)std::min<long long>(p.n_units, resident);
     void* args[] = {&p};

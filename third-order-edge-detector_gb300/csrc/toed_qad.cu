@@ -28,6 +28,7 @@
 //      the output record; in HYBRID precision the records whose vector nearly
 //      cancels are first contracted again in FP64 by the whole warp.
 #include "toed_common.cuh"
+#include "toed_edgel.cuh"
 #include "toed_internal.h"
 
 namespace toed {
@@ -297,8 +298,9 @@ __global__ void __launch_bounds__(kQadThreads, 3) fin_scatter_qad(const __grid_c
     for (int r0 = wid * 32; r0 < total; r0 += kQadThreads) {
         // lane e locates record r0 + e (list position, staging slot) and its
         // subpixel point pos = 2 x_out + 1 on the 2x grid (cpu_toed.cpp:516)
-        int my_d = -1, mX1 = 0, mY1 = 0;
-        long long my_src = 0;
+        int my_d = -1, mX1 = 0, mY1 = 0, my_gi = 0;
+        double2 my_xy = make_double2(0.0, 0.0);
+        float my_str = 0.f;
         float mtx = 0.f, mty = 0.f;
         if (r0 + lane < total) {
             const int r = r0 + lane;
@@ -309,7 +311,13 @@ __global__ void __launch_bounds__(kQadThreads, 3) fin_scatter_qad(const __grid_c
             }
             const long long d = base + r, src = (long long)s_src[lo] + (r - s_dst[lo]);
             if (d < cap && src < p.sc.staging_cap) {
-                const double2 xy = det_xy(det_stage(p.sc)[src], p.sc.staging_idx[src], 2 * im.W, p.hyb != 0);
+                const Staged e = load_staged(p.sc, src);
+                my_gi = e.idx;
+                const int Gr = e.idx / (2 * im.W);
+                const Fitted ft = fit_edgel(e, e.gx, e.gy, false, p.hyb != 0, Gr, e.idx - Gr * 2 * im.W);
+                my_xy = make_double2(ft.x, ft.y);
+                my_str = ft.str;
+                const double2 xy = my_xy;
                 const double px = 2.0 * xy.x + 1.0, py = 2.0 * xy.y + 1.0;
                 const double fpx = floor(px), fpy = floor(py);
                 mX1 = (int)fpx;
@@ -317,7 +325,6 @@ __global__ void __launch_bounds__(kQadThreads, 3) fin_scatter_qad(const __grid_c
                 mtx = (float)(px - fpx);
                 mty = (float)(py - fpy);
                 my_d = (int)d;
-                my_src = src;
             }
         }
         const int ne = min(32, total - r0);
@@ -369,9 +376,6 @@ __global__ void __launch_bounds__(kQadThreads, 3) fin_scatter_qad(const __grid_c
 #pragma unroll
         for (int q = 0; q < 9; ++q) mine[q] = sDer[wid][lane * 9 + q];
         __syncwarp();  // the next group overwrites the slots
-        const float4 my_st = my_d >= 0 ? det_stage(p.sc)[my_src] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const int my_gi = my_d >= 0 ? p.sc.staging_idx[my_src] : 0;
-        const double2 my_xy = my_d >= 0 ? det_xy(my_st, my_gi, 2 * im.W, p.hyb != 0) : make_double2(0.0, 0.0);
         // the third-order vector and the angle
         const float gx = mine[0], gy = mine[1], fxx = mine[2], fxy = mine[3], fyy = mine[4], fxxy = mine[5],
                     fxyy = mine[6], fxxx = mine[7], fyyy = mine[8];
@@ -413,15 +417,7 @@ __global__ void __launch_bounds__(kQadThreads, 3) fin_scatter_qad(const __grid_c
                               2.f * gx * gy * fxyy + gx * gx * fxxy + gy * gy * fyyy;
             ori = (tix == 0.f && tiy == 0.f) ? __int_as_float(0x7fc00000) : atan2f(tix, -tiy);
         }
-        if (my_d < 0) continue;
-        if (p.out_f64) {
-            double2* o = reinterpret_cast<double2*>(im.out) + 2 * my_d;
-            o[0] = my_xy;
-            o[1] = make_double2((double)ori, (double)my_st.w);
-        } else {
-            reinterpret_cast<float4*>(im.out)[my_d] = make_float4((float)my_xy.x, (float)my_xy.y, ori, my_st.w);
-        }
-        if (im.index) im.index[my_d] = my_gi;
+        if (my_d >= 0) write_edgel(p, im, my_d, my_xy.x, my_xy.y, ori, my_str, my_gi);
     }
 }
 

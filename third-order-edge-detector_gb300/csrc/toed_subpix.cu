@@ -1184,6 +1184,7 @@ cudaError_t subpix_launch(const toed_edgemap* maps, int n, const toed_subpix_par
     std::unique_ptr<BatchParams> bguard(b);
     b->n_img = n;
     b->n_tiles = p->n_seg_tiles;
+    b->seg_tile = kSegTile;
     b->out_f64 = p->out_f64;
     b->sc = s.sc;
     for (int i = 0; i < n; ++i) {
@@ -1198,7 +1199,7 @@ cudaError_t subpix_launch(const toed_edgemap* maps, int n, const toed_subpix_par
         d.H = p->m[i].h;
         d.W = p->m[i].w;
     }
-    if (e == cudaSuccess) e = launch_finalize(*b, stream);
+    if (e == cudaSuccess) e = launch_finalize_subpix(*b, stream);
     bool dense = false;
     for (int i = 0; i < n; ++i) dense = dense || maps[i].TO_E || maps[i].TO_O;
     if (dense && e == cudaSuccess) {
