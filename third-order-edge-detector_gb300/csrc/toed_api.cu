@@ -164,7 +164,7 @@ struct toed_ctx {
     double* sp_work = nullptr;  // TO correction at interp_n > 0: maps resized onto the work grid
     long long sp_work_cap = 0;
     int blocks_per_sm[TOED_MAX_RADIUS + 1][2] = {};  // [radius][corrected normal]
-    bool edgels_ready[TOED_MAX_RADIUS + 1] = {};     // the edgel kernel's attributes are set
+    bool edgels_ready[TOED_MAX_RADIUS + 1][2] = {};  // [radius][QaD]: the edgel kernel's attributes are set
     // launch shape chosen by toed_autotune per (radius, precision, size class of
     // the launch: floor(log2(pixels))); strip_rows 0 = heuristic
     toed_tuning tune[TOED_MAX_RADIUS + 1][2][kSizeClasses] = {};
@@ -424,9 +424,10 @@ static toed_status detect_chunk(toed_ctx* c, const toed_image* images, int n, co
         if (bps <= 0) return TOED_ERR_UNSUPPORTED;
     }
     const long long resident = (long long)bps * c->num_sms;
-    if (!c->edgels_ready[r]) {
-        TOED_CU(prepare_edgels(r));
-        c->edgels_ready[r] = true;
+    const bool qad = prm->orientation == TOED_ORI_QAD;
+    if (!c->edgels_ready[r][qad]) {
+        TOED_CU(prepare_edgels(r, qad));
+        c->edgels_ready[r][qad] = true;
     }
 
     BatchParams* p = new BatchParams();
@@ -449,7 +450,7 @@ static toed_status detect_chunk(toed_ctx* c, const toed_image* images, int n, co
     p->out_f64 = (prm->out_dtype == TOED_F64) ? 1 : 0;
     p->radius = r;
     p->hyb = hyb ? 1 : 0;
-    p->qad = prm->orientation == TOED_ORI_QAD ? 1 : 0;
+    p->qad = qad ? 1 : 0;
     p->nms_to = nmsto ? 1 : 0;
     p->ready = c->hb_ready;
     p->ready_epoch = c->hb_epoch;
@@ -469,7 +470,7 @@ static toed_status detect_chunk(toed_ctx* c, const toed_image* images, int n, co
     long long units = 0, tiles = 0, staging = 0, segs = 0, ed = 0;
     p->ed_rows = plan_ed_rows(images, n, c->num_sms);
     for (int i = 0; i < n; ++i) segs += 2LL * images[i].height * ((images[i].width + kInner - 1) / kInner);
-    const int seg_tile = p->seg_tile = p->qad ? kSegTile : plan_seg_tile(segs);
+    const int seg_tile = p->seg_tile = plan_seg_tile(segs);
     for (int i = 0; i < n; ++i) {
         const toed_image& im = images[i];
         DetImage& d = p->img[i];

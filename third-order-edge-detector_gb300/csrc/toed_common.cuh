@@ -63,7 +63,7 @@ constexpr int kWords = 8;  // scratch words: [0] queue [1] cursor [2] flags [3] 
 // window of kExt outputs at radius r, up to three floats of alignment before
 // it and one past an odd window's last pair.
 // An odd number of 16-byte groups: eight rows apart before a column meets its bank again.
-constexpr int staged_width(int r) { return ((kExt + 2 * r + 2 + 4 + (r & 1) + 3) / 4 | 1) * 4; }
+__host__ __device__ constexpr int staged_width(int r) { return ((kExt + 2 * r + 2 + 4 + (r & 1) + 3) / 4 | 1) * 4; }
 
 // 1-D taps, index k <-> offset x = k - (r+1) (+0.5 for the shifted set).
 // Filters: 0 G, 1 Gx, 2 Gxx, 3 Gxxx, 4..7 the same shifted by +0.5.

@@ -1,8 +1,7 @@
-// toed_finalize.cu -- ordering pass of the TO correction and of the
-// quick-and-dirty orientation mode: turns staged edgels and the row-segment
-// table into each image's edgel list in the reference's order (row-major,
-// cpu_toed.cpp:510-538).  (The detection's other modes are ordered by the
-// edgel kernel itself, toed_edgels.cu.)
+// toed_finalize.cu -- ordering pass of the TO correction: turns staged edgels
+// and the row-segment table into each map's edgel list in row-major order
+// (the detection's lists are ordered by toed_edgels.cu); and the copy of
+// finished lists to mapped host memory.
 //
 // Segments are (row, strip column) pairs laid out row-major per image and
 // padded to whole tiles of kSegTile.  Three short kernels:
@@ -159,37 +158,12 @@ cudaError_t launch_list_copy(const ListCopy* lists, int n, int rec, cudaStream_t
     return cudaSuccess;
 }
 
-cudaError_t preload_finalize(int radius, bool qad)
-{
-    if (!qad) return preload_edgels(radius);
-    cudaFuncAttributes fa;
-    cudaError_t e = cudaFuncGetAttributes(&fa, (const void*)fin_tile_sums);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)fin_tile_scan);
-    if (e == cudaSuccess) e = preload_scatter_qad(radius);
-    return e;
-}
-
-// Tile sums and their scan over the whole launch.
-static cudaError_t launch_tile_scan(const BatchParams& p, cudaStream_t stream)
+cudaError_t launch_finalize_subpix(const BatchParams& p, cudaStream_t stream)
 {
     void* args[] = {const_cast<BatchParams*>(&p)};
     cudaError_t e = cudaLaunchKernel((const void*)fin_tile_sums, dim3(p.n_tiles), dim3(256), args, 0, stream);
     if (e == cudaSuccess) e = cudaLaunchKernel((const void*)fin_tile_scan, dim3(1), dim3(1024), args, 0, stream);
-    return e;
-}
-
-cudaError_t launch_finalize(const BatchParams& p, cudaStream_t stream)
-{
-    if (!p.qad) return launch_edgels(p, stream);
-    const cudaError_t e = launch_tile_scan(p, stream);
-    return e == cudaSuccess ? launch_scatter_qad(p, stream) : e;
-}
-
-cudaError_t launch_finalize_subpix(const BatchParams& p, cudaStream_t stream)
-{
-    const cudaError_t e = launch_tile_scan(p, stream);
     if (e != cudaSuccess) return e;
-    void* args[] = {const_cast<BatchParams*>(&p)};
     return cudaLaunchKernel((const void*)fin_scatter, dim3(p.n_tiles), dim3(kFinThreads), args, 0, stream);
 }
 

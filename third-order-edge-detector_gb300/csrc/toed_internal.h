@@ -21,9 +21,9 @@ DetectEntry detect_entry(int radius, bool nmsto = false);
 // correction's kernels: the edgel lists.
 cudaError_t launch_finalize(const BatchParams& p, cudaStream_t stream);
 cudaError_t launch_finalize_subpix(const BatchParams& p, cudaStream_t stream);
-cudaError_t launch_edgels(const BatchParams& p, cudaStream_t stream);
-cudaError_t preload_edgels(int radius);
-cudaError_t prepare_edgels(int radius);  // its attributes, once per device and radius
+cudaError_t prepare_edgels(int radius, bool qad);  // the edgel kernel's attributes, once per device, radius and mode
+cudaError_t prepare_qad(int radius);
+cudaError_t launch_qad(const BatchParams& p, cudaStream_t stream);
 
 // One finished list from device memory to its mapped host buffers
 // (toed_finalize.cu): min(count, cap) records of `rec` bytes, the grid
@@ -44,10 +44,6 @@ cudaError_t preload_list_copy();
 // which must not happen while a detection launch waits for copies that the
 // host has yet to enqueue.
 cudaError_t preload_finalize(int radius, bool qad);
-// The ordering pass's last kernel in the TOED_ORI_QAD orientation mode (toed_qad.cu).
-cudaError_t launch_scatter_qad(const BatchParams& p, cudaStream_t stream);
-cudaError_t preload_scatter_qad(int radius);
-
 // The taps of (sigma, r) in FP64, and each rounded once to FP32; BatchParams::ytap from the latter.
 void make_taps64(double sigma, int r, TapBlock64* tb);
 void make_taps(double sigma, int r, TapBlock* tb);

@@ -93,7 +93,7 @@ cudaError_t device_setup(int dev, int r, bool nmsto, const DetectEntry& ent, uns
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ent.func, kThreads, ent.smem);
         if (e != cudaSuccess) return e;
         if (n <= 0) return cudaErrorInvalidConfiguration;
-        e = prepare_edgels(r);
+        for (int qad = 0; qad < 2 && e == cudaSuccess; ++qad) e = prepare_edgels(r, qad != 0);
         if (e != cudaSuccess) return e;
         b = n;
     }
