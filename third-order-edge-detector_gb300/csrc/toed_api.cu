@@ -395,13 +395,13 @@ static int plan_strip_rows(const toed_image* images, int n, long long resident)
 static int plan_seg_tile(long long nseg) { return nseg > 1024LL * kSegTile ? kScanTileMax : kSegTile; }
 
 // Image rows of an edgel-kernel tile: as tall as possible (a tile's pixels
-// include 2r + 2 rows of halo) while every SM still gets several tiles.
+// include 2r + 2 rows of halo) while every SM still gets its three CTAs.
 static int plan_ed_rows(const toed_image* images, int n, int num_sms)
 {
     long long rows = 0;  // strip rows of the launch
     for (int i = 0; i < n; ++i) rows += (long long)((images[i].width + kInner - 1) / kInner) * images[i].height;
     int t = kEdRowsMax;
-    while (t > 16 && rows < (long long)t * 8 * num_sms) t /= 2;
+    while (t > 16 && rows < (long long)t * 3 * num_sms) t /= 2;
     return t;
 }
 

@@ -277,6 +277,33 @@ inline cudaError_t launch_after(const void* func, dim3 grid, dim3 block, void** 
     return cudaLaunchKernelExC(&cfg, func, args);
 }
 
+// Four 8-bit pixels of a row at once: lane l of 16 takes the 4-byte aligned
+// word l of the row from column x0 on.  `c` is the word's first column less x0
+// (-3..0 for l = 0); bytes outside the image (or the word, where it is not
+// wholly inside the row) read as zero.
+struct Bytes4 {
+    unsigned w;
+    int c;
+};
+__device__ __forceinline__ Bytes4 fetch_bytes(const void* src, long long pitch, int H, int W, int y, int x0, int l, int n)
+{
+    const unsigned char* row = static_cast<const unsigned char*>(src) + (long long)y * pitch + x0;
+    Bytes4 b;
+    b.c = 4 * l - (int)(reinterpret_cast<uintptr_t>(row) & 3u);
+    b.w = 0u;
+    const int x = x0 + b.c;
+    if ((unsigned)y < (unsigned)H && b.c < n) {
+        if (x >= 0 && x + 3 < W) {
+            b.w = __ldg(reinterpret_cast<const unsigned*>(row + b.c));
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if ((unsigned)(x + e) < (unsigned)W) b.w |= (unsigned)__ldg(row + b.c + e) << (8 * e);
+        }
+    }
+    return b;
+}
+
 // x rounded down to a multiple of 4 (floats: 16 bytes, where a TMA box may start).
 __device__ __forceinline__ int floor4(int x) { return x >= 0 ? x & ~3 : -((3 - x) & ~3); }
 

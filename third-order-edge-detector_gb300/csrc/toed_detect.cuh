@@ -96,14 +96,11 @@ struct Cfg {
     static constexpr int MINB = smem <= 74 * 1024 ? 3 : 2;
 };
 
-// Image pixel as FP32 with zero padding outside the image (cpu_toed.cpp:207-208).
-__device__ __forceinline__ float fetch_px(const void* src, long long pitch, int H, int W, int dtype,
-                                          int y, int x)
+// Image pixel with zero padding outside the image (cpu_toed.cpp:207-208).
+__device__ __forceinline__ float fetch_px(const float* src, long long pitch, int H, int W, int y, int x)
 {
     if ((unsigned)y >= (unsigned)H || (unsigned)x >= (unsigned)W) return 0.f;
-    const long long o = (long long)y * pitch + x;
-    if (dtype == TOED_U8) return (float)__ldg((const unsigned char*)src + o);
-    return __ldg((const float*)src + o);
+    return __ldg(src + (long long)y * pitch + x);
 }
 
 // Ring row of x for 0 <= x < 2 * N (every ring index the kernel forms).
@@ -379,7 +376,8 @@ static __device__ __noinline__ bool wait_ready(const int* flag, int epoch, int s
 // Input rows: by TMA (DetImage::tma; float32 with 16-byte aligned rows), boxes
 // of 16 rows up to three ahead in a ring of three buffers that the row pass
 // reads in place; otherwise every warp loads the two rows of a box that it
-// alone reads, one box ahead in registers, and converts them.  Either way the
+// alone reads, one box ahead in registers (8-bit rows a word a lane), and
+// converts them.  Either way the
 // rows need no barrier of their own: two per step are left, row pass -> column
 // pass and column pass -> NMS (six when rows were converted into a ring and
 // the points listed for the whole CTA).
@@ -393,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<R, NMSTO>::MINB)
     static_assert(kThreads / 32 == 8 && kExt == 32, "column pass: one warp per (sub-grid, 8-row group)");
     static_assert(kThreads == B * (kExt / 2), "row pass: a thread per (row, column pair), a warp per two rows");
     static_assert(C::WROWS == 4, "NMS: four 2x-grid rows per warp");
-    static_assert(C::NIN <= 64, "a row's window: two floats per lane");
+    static_assert(C::NIN + 3 <= 64, "a row's window: two floats a lane, or four bytes a half-warp's lane");
     extern __shared__ __align__(128) unsigned char smem[];
     float* sRaw = reinterpret_cast<float*>(smem + C::off_raw);
     float2* sP = reinterpret_cast<float2*>(smem + C::off_P);
@@ -498,13 +496,22 @@ __global__ void __launch_bounds__(kThreads, Cfg<R, NMSTO>::MINB)
                 ib = ib + 1 == C::NBUF ? 0 : ib + 1;
             }
         };
-        // this warp's two rows of box q, columns lane and lane + 32, zero outside the image
+        // this warp's two rows of box q, zero outside the image: float32, columns
+        // lane and lane + 32 of both; 8 bits, four columns of one a lane
+        const bool u8 = dtype == TOED_U8;
         float pre[4];
+        Bytes4 pre8;
         auto fetch = [&](int q) {
+            if (u8) {
+                pre8 = fetch_bytes(src, pitch, H, W, row0(q) + 2 * wid + (lane >> 4), xin, lane & 15, C::NIN);
+            } else {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int c = lane + 32 * (e & 1);
-                pre[e] = c < C::NIN ? fetch_px(src, pitch, H, W, dtype, row0(q) + 2 * wid + (e >> 1), xin + c) : 0.f;
+                for (int e = 0; e < 4; ++e) {
+                    const int c = lane + 32 * (e & 1);
+                    pre[e] = c < C::NIN ? fetch_px(static_cast<const float*>(src), pitch, H, W,
+                                                   row0(q) + 2 * wid + (e >> 1), xin + c)
+                                        : 0.f;
+                }
             }
         };
         if (tma) {
@@ -536,9 +543,10 @@ __global__ void __launch_bounds__(kThreads, Cfg<R, NMSTO>::MINB)
                     __syncwarp();
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        const int c = lane + 32 * (e & 1);
-                        if (c < C::NIN && TOED_IN_BOUNDS(shift + c < C::BW, p.sc.words))
-                            box[(2 * wid + (e >> 1)) * C::BW + shift + c] = pre[e];
+                        const int c = u8 ? pre8.c + e : lane + 32 * (e & 1);
+                        const int row = 2 * wid + (u8 ? lane >> 4 : e >> 1);
+                        if ((unsigned)c < (unsigned)C::NIN && TOED_IN_BOUNDS(shift + c < C::BW, p.sc.words))
+                            box[row * C::BW + shift + c] = u8 ? (float)((pre8.w >> (8 * e)) & 255u) : pre[e];
                     }
                     __syncwarp();
                     if (q + 1 < nbox) fetch(q + 1);

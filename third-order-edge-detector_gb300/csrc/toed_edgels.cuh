@@ -469,21 +469,28 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
         }
     } else {
         const int nr = nrow + 2 * E::HALO;
-        constexpr int NC = (E::TW + 31) / 32;
+        if (im.dtype == TOED_U8) {  // a word a lane, two rows a warp
+            static_assert(E::TW + 3 <= 64, "sixteen words a row");
 #pragma unroll 4
-        for (int r = wid; r < nr; r += kEdThreads / 32) {
+            for (int r0 = 2 * wid; r0 < nr; r0 += 2 * (kEdThreads / 32)) {
+                const int r = r0 + (lane >> 4);
+                const Bytes4 b = fetch_bytes(im.src, im.pitch, H, W, py + r, px, lane & 15, E::TW);
 #pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                const int col = lane + 32 * c;
-                if (col < E::TW) {
-                    const int y = py + r, x = px + col;
-                    float v = 0.f;
-                    if ((unsigned)y < (unsigned)H && (unsigned)x < (unsigned)W) {
-                        const long long o = (long long)y * im.pitch + x;
-                        v = im.dtype == TOED_U8 ? (float)__ldg(static_cast<const unsigned char*>(im.src) + o)
-                                                : __ldg(static_cast<const float*>(im.src) + o);
-                    }
-                    sPix[r * TP + shift + col] = v;
+                for (int e = 0; e < 4; ++e)
+                    if (r < nr && (unsigned)(b.c + e) < (unsigned)E::TW)
+                        sPix[r * TP + shift + b.c + e] = (float)((b.w >> (8 * e)) & 255u);
+            }
+        } else {
+            const float* src = static_cast<const float*>(im.src);
+#pragma unroll 4
+            for (int r = wid; r < nr; r += kEdThreads / 32) {
+#pragma unroll
+                for (int c = 0; c < (E::TW + 31) / 32; ++c) {
+                    const int col = lane + 32 * c, y = py + r, x = px + col;
+                    if (col < E::TW)
+                        sPix[r * TP + shift + col] = (unsigned)y < (unsigned)H && (unsigned)x < (unsigned)W
+                                                         ? __ldg(src + (long long)y * im.pitch + x)
+                                                         : 0.f;
                 }
             }
         }
