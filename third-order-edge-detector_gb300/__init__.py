@@ -327,7 +327,7 @@ class Detector:
             })
         return outs
 
-    def _image_struct(self, img, out):
+    def _image_dtype(self, img):
         t = self.torch
         if img.dim() != 2 or img.device.type != "cuda":
             raise ValueError("images must be 2-D CUDA tensors")
@@ -339,6 +339,10 @@ class Detector:
             raise ValueError("image dtype must be uint8 or float32")
         if img.stride(1) != 1:
             raise ValueError("image rows must be contiguous")
+        return dt
+
+    def _image_struct(self, img, out):
+        dt = self._image_dtype(img)
         H, W = img.shape
         return toed_image(img.data_ptr(), H, W, img.stride(0), dt, out["edgels"].data_ptr(),
                           out["capacity"], out["count"].data_ptr(),
@@ -434,19 +438,39 @@ class Detector:
         dicts with ``edgels`` (N x 4: x, y, orientation, strength) and,
         with ``index``, the 2x-grid linear index of each edgel."""
         p = make_params(sigma, radius, threshold, border, out_dtype, precision, orientation, nms_direction)
-        outs = self.alloc_outputs([tuple(im.shape) for im in images], capacity, out_dtype, index)
-        self.detect_into(images, outs, p, stream)
-        s = stream if stream is not None else self.torch.cuda.current_stream(self.device)
+        t = self.torch
+        dts = [self._image_dtype(im) for im in images]
+        caps = [int(capacity) if capacity is not None else 4 * im.shape[0] * im.shape[1] for im in images]
+        # one buffer of each kind for the batch, and one read of all its counts:
+        # per-image buffers and reads cost 30 us an image of host time
+        edgels, idx, counts = self._flat_lists(caps, out_dtype, index)
+        arr, at = (toed_image * len(images))(), 0
+        pe, pi, pc, rec = edgels.data_ptr(), idx.data_ptr() if index else 0, counts.data_ptr(), 4 * edgels.element_size()
+        for k, (im, dt, cap) in enumerate(zip(images, dts, caps)):
+            H, W = im.shape
+            arr[k] = toed_image(im.data_ptr(), H, W, im.stride(0), dt, pe + at * rec, cap, pc + 4 * k,
+                                pi + 4 * at if index else None)
+            at += max(cap, 1)
+        s = stream if stream is not None else t.cuda.current_stream(self.device)
+        _check(lib().toed_detect_batch(self._ctx, arr, len(images), ctypes.byref(p), ctypes.c_void_p(s.cuda_stream)),
+               "toed_detect_batch")
         s.synchronize()
-        res = []
-        for o in outs:
-            n = int(o["count"].item())
-            m = min(n, o["capacity"])
-            r = {"count": n, "edgels": o["edgels"][:m]}
+        res, at = [], 0
+        for n, cap in zip(counts.tolist(), caps):
+            m = min(n, cap)
+            r = {"count": n, "edgels": edgels[at:at + m]}
             if index:
-                r["index"] = o["index"][:m]
+                r["index"] = idx[at:at + m]
             res.append(r)
+            at += max(cap, 1)
         return res
+
+    def _flat_lists(self, caps, out_dtype, index=True):
+        """Edgel, index and count buffers of a whole batch (the library writes every count)."""
+        t, dev, total = self.torch, f"cuda:{self.device}", sum(max(c, 1) for c in caps)
+        return (t.empty((total, 4), dtype=t.float64 if out_dtype == TOED_F64 else t.float32, device=dev),
+                t.empty(total, dtype=t.int32, device=dev) if index else None,
+                t.empty(len(caps), dtype=t.int32, device=dev))
 
     def detect(self, image, **kw):
         return self.detect_batch([image], **kw)[0]
@@ -456,18 +480,28 @@ class Detector:
         """Adjoint of detect_batch with the selection frozen: given the
         forward's images, its per-image grid indices and dL/d(edgels)
         (N x 4 each), returns (dL/dimages as float32 tensors, dL/dsigma)."""
+        grads, gs, _ = self._adjoint(images, indices, grad_edgels, sigma, radius, out_dtype, stream)
+        return grads, gs
+
+    def _adjoint(self, images, indices, grad_edgels, sigma, radius, out_dtype=TOED_F32, stream=None):
+        """backward_batch; the third value is the (n, H, W) buffer that images
+        of one size share for their gradients, or None."""
         t = self.torch
-        dev = f"cuda:{self.device}"
+        dev = t.device("cuda", self.device)
         items, grads = [], []
         gdt = t.float64 if out_dtype == TOED_F64 else t.float32
         keep = []
-        for im, idx, ge in zip(images, indices, grad_edgels):
+        same = len(images) > 0 and all(im.shape == images[0].shape for im in images)
+        flat = t.empty((len(images), *images[0].shape), dtype=t.float32, device=dev) if same else None
+        for k, (im, idx, ge) in enumerate(zip(images, indices, grad_edgels)):
             if im.stride(1) != 1:
                 raise ValueError("image rows must be contiguous")
             H, W = im.shape
-            gi = idx.to(device=dev, dtype=t.int32).contiguous()
-            go = ge.to(device=dev, dtype=gdt).contiguous()
-            gp = t.empty((H, W), dtype=t.float32, device=dev)
+            gi = idx if idx.dtype == t.int32 and idx.device == dev and idx.is_contiguous() else \
+                idx.to(device=dev, dtype=t.int32).contiguous()
+            go = ge if ge.dtype == gdt and ge.device == dev and ge.is_contiguous() else \
+                ge.to(device=dev, dtype=gdt).contiguous()
+            gp = flat[k] if same else t.empty((H, W), dtype=t.float32, device=dev)
             keep += [gi, go]
             grads.append(gp)
             items.append(toed_grad_image(im.data_ptr(), H, W, im.stride(0),
@@ -480,7 +514,7 @@ class Detector:
         s = stream if stream is not None else t.cuda.current_stream(self.device)
         _check(lib().toed_backward_batch(self._ctx, arr, len(items), ctypes.byref(p), ctypes.c_void_p(gs.data_ptr()),
                                          ctypes.c_void_p(s.cuda_stream)), "toed_backward_batch")
-        return grads, gs
+        return grads, gs, flat
 
     def subpix_to_correct_batch(self, maps, thresh=0.2, sigma=2.0, nbr_radius=2.0, thetas=None,
                                 out_dtype=TOED_F32, precision=TOED_HYBRID, capacity=None, dense=True,
@@ -494,6 +528,14 @@ class Detector:
         dt = t.float64 if out_dtype == TOED_F64 else t.float32
         dev = f"cuda:{self.device}"
         arr, outs = [], []
+        caps = [int(capacity) if capacity is not None
+                else ((E.shape[0] - 1) * (1 << interp_n) + 1) * ((E.shape[1] - 1) * (1 << interp_n) + 1)
+                for E in maps if E.dim() == 2]
+        if len(caps) != len(maps):
+            raise ValueError("edge maps must be 2-D row-contiguous float32/float64 CUDA tensors")
+        edgels, _, counts = self._flat_lists(caps, out_dtype, False)
+        dense_buf = t.empty(2 * sum(E.numel() for E in maps), dtype=dt, device=dev) if dense else None
+        at = dense_at = 0
         for k, E in enumerate(maps):
             if E.dim() != 2 or E.dtype not in (t.float32, t.float64) or E.stride(1) != 1:
                 raise ValueError("edge maps must be 2-D row-contiguous float32/float64 CUDA tensors")
@@ -501,16 +543,17 @@ class Detector:
             if th is not None and (th.dtype != E.dtype or th.stride() != E.stride() or th.shape != E.shape):
                 raise ValueError("orientation map must match the edge map's dtype, shape and strides")
             h, w = E.shape
-            cap = int(capacity) if capacity is not None else ((h - 1) * (1 << interp_n) + 1) * ((w - 1) * (1 << interp_n) + 1)
-            o = {"edgels": t.empty((max(cap, 1), 4), dtype=dt, device=dev),
-                 "count": t.zeros(1, dtype=t.int32, device=dev), "capacity": cap}
+            cap = caps[k]
+            o = {"edgels": edgels[at:at + max(cap, 1)], "capacity": cap}
+            at += max(cap, 1)
             if dense:
-                o["TO_E"] = t.empty((h, w), dtype=dt, device=dev)
-                o["TO_O"] = t.empty((h, w), dtype=dt, device=dev)
+                for name in ("TO_E", "TO_O"):
+                    o[name] = dense_buf[dense_at:dense_at + h * w].view(h, w)
+                    dense_at += h * w
             outs.append(o)
             arr.append(toed_edgemap(E.data_ptr(), th.data_ptr() if th is not None else None, h, w,
                                     E.stride(0), TOED_F64 if E.dtype == t.float64 else TOED_F32,
-                                    o["edgels"].data_ptr(), cap, o["count"].data_ptr(),
+                                    o["edgels"].data_ptr(), cap, counts.data_ptr() + 4 * k,
                                     o["TO_E"].data_ptr() if dense else None,
                                     o["TO_O"].data_ptr() if dense else None))
         a = (toed_edgemap * len(arr))(*arr)
@@ -521,8 +564,7 @@ class Detector:
                                                   ctypes.c_void_p(s.cuda_stream)), "toed_subpix_to_correct_batch")
         s.synchronize()
         res = []
-        for o in outs:
-            n = int(o["count"].item())
+        for n, o in zip(counts.tolist(), outs):
             r = {"count": n, "edgels": o["edgels"][:min(n, o["capacity"])]}
             if dense:
                 r["TO_E"], r["TO_O"] = o["TO_E"], o["TO_O"]
@@ -700,8 +742,8 @@ def differentiable_detect(images, sigma, threshold=2.0, radius=0, detector=None)
         def backward(ctx, g_edg, g_idx, g_cnt):
             (imgs,) = ctx.saved_tensors
             splits = torch.split(g_edg.contiguous(), ctx.counts)
-            grads, gs = det.backward_batch(list(imgs), ctx.idx, list(splits), sigma=ctx.sigma, radius=radius)
-            gi = torch.stack(grads) if ctx.needs_input_grad[0] else None
+            _, gs, flat = det._adjoint(list(imgs), ctx.idx, list(splits), ctx.sigma, radius)
+            gi = flat if ctx.needs_input_grad[0] else None
             gsig = gs.reshape(()).to(dtype=ctx.sig_meta[0], device=ctx.sig_meta[1]) if ctx.needs_input_grad[1] else None
             return gi, gsig
 
