@@ -13,19 +13,19 @@
 //                   along dir on E with the parabola fit (:413-519); edgels are
 //                   compacted in row-major order into staging with a
 //                   (row, tile column) segment table and a per-pixel id map.
+//   tc_isolate      per segment: an edgel survives if another lies within
+//                   the neighbour radius in the reference's 3x3 cell grid
+//                   (:563-621), found through the id map.
 //   tc_correct      one CTA per tile that holds edgels: the eight circular
 //                   separable Gaussian-derivative convolutions (:377-411,
 //                   :641-648) fused over the tile + halo in shared memory
 //                   (6 row filters, 8 column filters), then per edgel the Keys
 //                   bicubic samples of ten planes (:521-556) and the corrected
 //                   orientation (:663-694).
-//   tc_isolate      per segment: an edgel survives if another lies within
-//                   the neighbour radius in the reference's 3x3 cell grid
-//                   (:563-621), found through the id map.
 //   tc_compact      per segment: stable in-place compaction of survivors.
-//   then the ordering pass of toed_finalize.cu, and tc_dense (two passes)
-//   for the dense TO_E / TO_O maps at round(x, y), later edgels winning
-//   (:708-715).
+//   then the ordering pass of toed_finalize.cu; the dense TO_E / TO_O maps at
+//   round(x, y), later edgels winning (:708-715), by tc_dense_gather before
+//   the compaction, at interp_n > 0 by tc_dense (two passes) at the end.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -195,17 +195,78 @@ __device__ __forceinline__ float2 tri_df(int k)
     }
 }
 
-__device__ __forceinline__ double cubic_w(double s)
-{  // Keys kernel, a = -0.5 (:57-67)
-    const double a = -0.5;
-    const double x = fabs(s);
-    if (x <= 1.0) return ((a + 2) * x - (a + 3)) * x * x + 1;
-    if (x < 2.0) return ((a * x - 5 * a) * x + 8 * a) * x - 4 * a;
-    return 0.0;
+// The same estimate in 64-bit integers, exact: the map scaled by a power of two
+// so that its largest value in the tile's region is below 2^49, every float down
+// to 2^-25 of it is a whole number (smaller ones are off by half a unit), the
+// triangle filter is a box of five of a box of five -- two running sums of
+// two additions an output instead of nine double-float products and sums --
+// and the second differences are whole numbers below 2^63.  Only the last step,
+// the division by 25^2 and the factor 1/4, is double-float.
+// Five-box sums over nine consecutive outputs: T[c] = sum_k (5 - |k|) v[c + 4 + k].
+__device__ __forceinline__ void triangle9(const long long (&v)[17], long long (&T)[9])
+{
+    long long b[13];
+    b[0] = v[0] + v[1] + v[2] + v[3] + v[4];
+#pragma unroll
+    for (int i = 1; i < 13; ++i) b[i] = b[i - 1] + v[i + 4] - v[i - 1];
+    T[0] = b[0] + b[1] + b[2] + b[3] + b[4];
+#pragma unroll
+    for (int i = 1; i < 9; ++i) T[i] = T[i - 1] + b[i + 4] - b[i - 1];
+}
+
+// n / 2500 * down (down a power of two) as a double-float.
+__device__ __forceinline__ float2 df_second(long long n, float down)
+{
+    constexpr double k = 1.0 / 2500.0;
+    constexpr float khi = (float)k, klo = (float)(k - (double)khi);
+    const float hi = __ll2float_rn(n);
+    const float lo = __ll2float_rn(n - __float2ll_rn(hi));
+    const float2 q = df_mul(make_float2(hi, lo), make_float2(khi, klo));
+    return make_float2(q.x * down, q.y * down);
+}
+
+// Four times the second differences of the smoothed map.
+struct Second {
+    long long xx, yy, xy;
+};
+// At pixels of a tile (corner i0, j0) on the map's border: gradient2 is one-sided there.
+__device__ __noinline__ Second second_border(const long long (*smoothed)[kT + 4], int i, int j, int h, int w, int i0, int j0)
+{
+    auto sm = [&](int y, int x) { return smoothed[y - i0 + 2][x - j0 + 2]; };
+    auto ox2 = [&](int y, int x) {
+        return (x == 0) ? 2 * (sm(y, 1) - sm(y, 0)) : (x == w - 1 ? 2 * (sm(y, x) - sm(y, x - 1)) : sm(y, x + 1) - sm(y, x - 1));
+    };
+    auto oy2 = [&](int y, int x) {
+        return (y == 0) ? 2 * (sm(1, x) - sm(0, x)) : (y == h - 1 ? 2 * (sm(y, x) - sm(y - 1, x)) : sm(y + 1, x) - sm(y - 1, x));
+    };
+    Second s;
+    s.xx = (j == 0) ? 2 * (ox2(i, 1) - ox2(i, 0)) : (j == w - 1 ? 2 * (ox2(i, j) - ox2(i, j - 1)) : ox2(i, j + 1) - ox2(i, j - 1));
+    s.xy = (j == 0) ? 2 * (oy2(i, 1) - oy2(i, 0)) : (j == w - 1 ? 2 * (oy2(i, j) - oy2(i, j - 1)) : oy2(i, j + 1) - oy2(i, j - 1));
+    s.yy = (i == 0) ? 2 * (oy2(1, j) - oy2(0, j)) : (i == h - 1 ? 2 * (oy2(i, j) - oy2(i - 1, j)) : oy2(i + 1, j) - oy2(i - 1, j));
+    return s;
+}
+
+// (cos, sin) of atan(y / x) wrapped to [0, pi) (:370-374, :296-305), x != 0:
+// th = atan(y / x) lies in (-pi/2, pi/2), so wrap_mod_pi (:216-222) adds pi
+// exactly when th < 0: (|x|, y sgn x) / |(x, y)|, negated when x y < 0.
+__device__ __forceinline__ float2 hessian_dir(float x, float y)
+{
+    const float rn = rsqrtf(fmaf(x, x, y * y));
+    const float cx = fabsf(x) * rn, sy = copysignf(1.f, x) * y * rn;
+    return (x * y < 0.f) ? make_float2(-cx, -sy) : make_float2(cx, sy);
+}
+// x = 0: pi / 2 after the wrap, NaN for 0 / 0 (as the reference).
+__device__ __noinline__ float2 hessian_dir0(float x, float y)
+{
+    float a2 = fmodf(atanf(y / x), 3.14159265358979323846f);
+    if (a2 < 0.f) a2 += 3.14159265358979323846f;
+    float sn, cs;
+    sincosf(a2, &sn, &cs);
+    return make_float2(cs, sn);
 }
 
 __device__ __forceinline__ float cubic_wf(float s)
-{  // the same kernel in FP32, for interpolation weights of FP32 data
+{  // Keys kernel, a = -0.5 (:57-67)
     const float a = -0.5f;
     const float x = fabsf(s);
     if (x <= 1.f) return ((a + 2.f) * x - (a + 3.f)) * x * x + 1.f;
@@ -213,12 +274,82 @@ __device__ __forceinline__ float cubic_wf(float s)
     return 0.f;
 }
 
+// A tile's orientation estimate in double-float arithmetic, where integers do
+// not do (tc_orient_nms): out of line, so that the common path's code fits the
+// instruction cache.
+constexpr int kHaloE = 6, kRegionE = kT + 2 * kHaloE;  // E region of a tile: rows/cols i0-6 .. i0+37
+static __device__ __noinline__ void orient_df(const SubParams& p, const SubMap& M, const float (*sE)[kRegionE + 1],
+                                              unsigned char* sStage, float2 (*sDir)[kT], int i0, int j0)
+{
+    constexpr int NE = kRegionE;
+    const int tid = threadIdx.x, h = M.h, w = M.w;
+    // the orientation estimate in double-float arithmetic (see
+    // df_two_sum); the same sums, in the same order, as the FP32 form
+    float2(*sTmpD)[kT + 4] = reinterpret_cast<float2(*)[kT + 4]>(sStage);          // cols j0-2 .. j0+33
+    float2(*sSmD)[kT + 4] = reinterpret_cast<float2(*)[kT + 4]>(sStage + sizeof(float2) * NE * (kT + 4));  // rows/cols -2 .. +33
+#pragma unroll 1
+    for (int q = tid; q < NE * (kT + 4); q += blockDim.x) {
+        const int a = q / (kT + 4), c = q - a * (kT + 4);
+        float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int qq = -kTriR; qq <= kTriR; ++qq)
+            acc = df_add(acc, df_mul_f(sE[a][c + 4 - qq], tri_df(qq)));
+        sTmpD[a][c] = acc;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int q = tid; q < (kT + 4) * (kT + 4); q += blockDim.x) {
+        const int d = q / (kT + 4), c = q - d * (kT + 4);
+        float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int pp = -kTriR; pp <= kTriR; ++pp) acc = df_add(acc, df_mul(sTmpD[d + 4 - pp][c], tri_df(pp)));
+        sSmD[d][c] = acc;
+    }
+    __syncthreads();
+    // gradient2 (:346-355) of the smoothed map and of its gradients, at
+    // the tile's pixels, one-sided at the image borders
+    auto sm = [&](int i, int j) { return sSmD[i - i0 + 2][j - j0 + 2]; };
+    auto ox = [&](int i, int j) {
+        return (j == 0) ? df_sub(sm(i, 1), sm(i, 0))
+                        : (j == w - 1 ? df_sub(sm(i, j), sm(i, j - 1)) : df_half(df_sub(sm(i, j + 1), sm(i, j - 1))));
+    };
+    auto oy = [&](int i, int j) {
+        return (i == 0) ? df_sub(sm(1, j), sm(0, j))
+                        : (i == h - 1 ? df_sub(sm(i, j), sm(i - 1, j)) : df_half(df_sub(sm(i + 1, j), sm(i - 1, j))));
+    };
+#pragma unroll 1
+    for (int q = tid; q < kT * kT; q += blockDim.x) {
+        const int a = q >> 5, b = q & 31;
+        const int i = i0 + a, j = j0 + b;
+        if (i >= h || j >= w) continue;
+        const float2 oxx = (j == 0) ? df_sub(ox(i, 1), ox(i, 0))
+                                    : (j == w - 1 ? df_sub(ox(i, j), ox(i, j - 1))
+                                                  : df_half(df_sub(ox(i, j + 1), ox(i, j - 1))));
+        const float2 oxy = (j == 0) ? df_sub(oy(i, 1), oy(i, 0))
+                                    : (j == w - 1 ? df_sub(oy(i, j), oy(i, j - 1))
+                                                  : df_half(df_sub(oy(i, j + 1), oy(i, j - 1))));
+        const float2 oyy = (i == 0) ? df_sub(oy(1, j), oy(0, j))
+                                    : (i == h - 1 ? df_sub(oy(i, j), oy(i - 1, j))
+                                                  : df_half(df_sub(oy(i + 1, j), oy(i - 1, j))));
+        // the sign of Oxy and x = Oxx + 1e-5 decided on the double-float values
+        const float sgn = (oxy.x < 0.f) ? 1.f : ((oxy.x > 0.f) ? -1.f : 0.f);
+        constexpr double kEps = 1e-5;
+        constexpr float kEpsHi = (float)kEps, kEpsLo = (float)(kEps - (double)kEpsHi);
+        const float2 xd = df_add(oxx, make_float2(kEpsHi, kEpsLo));
+        const float x = xd.x, y = oyy.x * sgn;
+        const float2 d = x != 0.f ? hessian_dir(x, y) : hessian_dir0(x, y);
+        sDir[a][b] = d;
+        p.dir[M.px_base + (long long)i * w + j] = d;
+    }
+    __syncthreads();
+}
+
 // ---------------------------------------------------------------------------
 // Orientation + NMS
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256, 5) tc_orient_nms(const __grid_constant__ SubParams p)
 {
-    constexpr int HE = 6, NE = kT + 2 * HE;  // E region: rows/cols i0-6 .. i0+37
+    constexpr int HE = kHaloE, NE = kRegionE;
     __shared__ float sE[NE][NE + 1];
     __shared__ float2 sDir[kT][kT];
     __shared__ int sRowCnt[kT], sRowOff[kT], sCandOff[kT + 1];
@@ -250,98 +381,105 @@ __global__ void __launch_bounds__(256, 5) tc_orient_nms(const __grid_constant__ 
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
 
     const bool inside = i0 - HE >= 0 && j0 - HE >= 0 && i0 - HE + NE <= h && j0 - HE + NE <= w;  // no padding
-    for (int q = tid; q < NE * NE; q += blockDim.x) {
-        const int a = q / NE, b = q - a * NE;
-        const int ii = inside ? i0 - HE + a : wrap_sym(i0 - HE + a, h);
-        const int jj = inside ? j0 - HE + b : wrap_sym(j0 - HE + b, w);
-        sE[a][b] = load_map(M.E, dtype, (long long)ii * M.pitch + jj);
-    }
-    __syncthreads();
-
+    const bool estimate = M.theta == nullptr && p.hyb;
     // HYBRID: tiles holding an NMS candidate (E > thresh inside the margin)
-    // estimate the orientation in double-float arithmetic; the others, whose
-    // directions only weight the Hx / Hy maps, in FP32
-    bool df_tile = false;
-    if (M.theta == nullptr && p.hyb) {
-        bool any = false;
-        for (int q = tid; q < kT * kT; q += blockDim.x) {
-            const int a = q >> 5, b = q & 31, i = i0 + a, j = j0 + b;
-            any = any || (i >= M.margin + 1 && i < h - M.margin - 2 && j >= M.margin + 1 && j < w - M.margin - 2 &&
-                          sE[a + HE][b + HE] > p.thresh);
+    // estimate the orientation beyond FP32; the others, whose directions only
+    // weight the Hx / Hy maps, in FP32
+    bool any = false;
+    unsigned top = 0u;  // largest |E| of the tile's region, as bits
+#pragma unroll 2
+    for (int a = wid; a < NE; a += 8) {  // a warp per row, lanes along it
+        const int i = i0 - HE + a, ii = inside ? i : wrap_sym(i, h);
+        const bool row = a >= HE && a < HE + kT && i >= M.margin + 1 && i < h - M.margin - 2;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int b = lane + 32 * c;
+            if (b < NE) {
+                const int j = j0 - HE + b, jj = inside ? j : wrap_sym(j, w);
+                const float v = load_map(M.E, dtype, (long long)ii * M.pitch + jj);
+                sE[a][b] = v;
+                top = max(top, __float_as_uint(v) & 0x7fffffffu);
+                any = any || (row && b >= HE && b < HE + kT && j >= M.margin + 1 && j < w - M.margin - 2 && v > p.thresh);
+            }
         }
-        df_tile = __syncthreads_or(any);
     }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0) sRowCnt[wid] = (int)top;
+    const bool df_tile = __syncthreads_or(any) && estimate;
     if (df_tile) {
-        // the orientation estimate in double-float arithmetic (see
-        // df_two_sum); the same sums, in the same order, as the FP32 form
-        float2(*sTmpD)[kT + 4] = reinterpret_cast<float2(*)[kT + 4]>(sStage);          // cols j0-2 .. j0+33
-        float2(*sSmD)[kT + 4] = reinterpret_cast<float2(*)[kT + 4]>(sStage + 2 * kTmpB);  // rows/cols -2 .. +33
-        for (int q = tid; q < NE * (kT + 4); q += blockDim.x) {
-            const int a = q / (kT + 4), c = q - a * (kT + 4);
-            float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int qq = -kTriR; qq <= kTriR; ++qq)
-                acc = df_add(acc, df_mul_f(sE[a][c + 4 - qq], tri_df(qq)));
-            sTmpD[a][c] = acc;
+        for (int u = 0; u < 8; ++u) top = max(top, (unsigned)sRowCnt[u]);
+    }
+    // integers where the candidates' own values (> thresh) are not small beside
+    // the largest of the region, so that half a unit is 2^-41 of theirs or less;
+    // double-floats otherwise, and where a value is not finite
+    const bool int_tile = df_tile && top < 0x7f800000u && __uint_as_float(top) <= 256.f * p.thresh &&
+                          __uint_as_float(top) > 1e-18f;  // (the scale is a normal float)
+    if (int_tile) {
+        long long(*sTmpI)[kT + 4] = reinterpret_cast<long long(*)[kT + 4]>(sStage);               // cols j0-2 .. j0+33
+        long long(*sSmI)[kT + 4] = reinterpret_cast<long long(*)[kT + 4]>(sStage + 2 * kTmpB);    // rows/cols -2 .. +33
+        const int ex = (int)(top >> 23) - 127;  // largest < 2^(ex + 1)
+        const float up = __int_as_float((48 - ex + 127) << 23), down = __int_as_float((ex - 48 + 127) << 23);
+        static_assert((kT + 4) % 9 == 0 && NE * ((kT + 4) / 9) <= 256, "an item a thread: nine outputs of a row or column");
+        if (tid < NE * 4) {
+            const int a = tid % NE, c0 = tid / NE * 9;
+            long long v[17], T[9];
+#pragma unroll
+            for (int u = 0; u < 17; ++u) v[u] = __float2ll_rn(sE[a][c0 + u] * up);
+            triangle9(v, T);
+#pragma unroll
+            for (int u = 0; u < 9; ++u) sTmpI[a][c0 + u] = T[u];
         }
         __syncthreads();
-        for (int q = tid; q < (kT + 4) * (kT + 4); q += blockDim.x) {
-            const int d = q / (kT + 4), c = q - d * (kT + 4);
-            float2 acc = make_float2(0.f, 0.f);
+        if (tid < (kT + 4) * 4) {
+            const int c = tid % (kT + 4), d0 = tid / (kT + 4) * 9;
+            long long v[17], T[9];
 #pragma unroll
-            for (int pp = -kTriR; pp <= kTriR; ++pp) acc = df_add(acc, df_mul(sTmpD[d + 4 - pp][c], tri_df(pp)));
-            sSmD[d][c] = acc;
+            for (int u = 0; u < 17; ++u) v[u] = sTmpI[d0 + u][c];
+            triangle9(v, T);
+#pragma unroll
+            for (int u = 0; u < 9; ++u) sSmI[d0 + u][c] = T[u];
         }
         __syncthreads();
-        // gradient2 (:346-355) of the smoothed map and of its gradients, at
-        // the tile's pixels, one-sided at the image borders
-        auto sm = [&](int i, int j) { return sSmD[i - i0 + 2][j - j0 + 2]; };
-        auto ox = [&](int i, int j) {
-            return (j == 0) ? df_sub(sm(i, 1), sm(i, 0))
-                            : (j == w - 1 ? df_sub(sm(i, j), sm(i, j - 1)) : df_half(df_sub(sm(i, j + 1), sm(i, j - 1))));
-        };
-        auto oy = [&](int i, int j) {
-            return (i == 0) ? df_sub(sm(1, j), sm(0, j))
-                            : (i == h - 1 ? df_sub(sm(i, j), sm(i - 1, j)) : df_half(df_sub(sm(i + 1, j), sm(i - 1, j))));
-        };
+        const bool inner = i0 >= 2 && j0 >= 2 && i0 + kT + 2 <= h && j0 + kT + 2 <= w;
+#pragma unroll 1
         for (int q = tid; q < kT * kT; q += blockDim.x) {
             const int a = q >> 5, b = q & 31;
             const int i = i0 + a, j = j0 + b;
             if (i >= h || j >= w) continue;
-            const float2 oxx = (j == 0) ? df_sub(ox(i, 1), ox(i, 0))
-                                        : (j == w - 1 ? df_sub(ox(i, j), ox(i, j - 1))
-                                                      : df_half(df_sub(ox(i, j + 1), ox(i, j - 1))));
-            const float2 oxy = (j == 0) ? df_sub(oy(i, 1), oy(i, 0))
-                                        : (j == w - 1 ? df_sub(oy(i, j), oy(i, j - 1))
-                                                      : df_half(df_sub(oy(i, j + 1), oy(i, j - 1))));
-            const float2 oyy = (i == 0) ? df_sub(oy(1, j), oy(0, j))
-                                        : (i == h - 1 ? df_sub(oy(i, j), oy(i - 1, j))
-                                                      : df_half(df_sub(oy(i + 1, j), oy(i - 1, j))));
-            // the sign of Oxy and x = Oxx + 1e-5 decided on the double-float values
-            const float sgn = (oxy.x < 0.f) ? 1.f : ((oxy.x > 0.f) ? -1.f : 0.f);
-            constexpr double kEps = 1e-5;
-            constexpr float kEpsHi = (float)kEps, kEpsLo = (float)(kEps - (double)kEpsHi);
-            const float2 xd = df_add(oxx, make_float2(kEpsHi, kEpsLo));
-            const float x = xd.x, y = oyy.x * sgn;
-            float2 d;
-            if (x != 0.f) {
-                // (cos, sin) of atan(y / x) wrapped to [0, pi) (:370-374, :296-305), as below
-                const float rn = rsqrtf(fmaf(x, x, y * y));
-                const float cx = fabsf(x) * rn, sy = copysignf(1.f, x) * y * rn;
-                d = (x * y < 0.f) ? make_float2(-cx, -sy) : make_float2(cx, sy);
-            } else {  // atan(y / 0): pi / 2 after the wrap, NaN for 0 / 0 (as the reference)
-                float a2 = fmodf(atanf(y / x), 3.14159265358979323846f);
-                if (a2 < 0.f) a2 += 3.14159265358979323846f;
-                float sn, cs;
-                sincosf(a2, &sn, &cs);
-                d = make_float2(cs, sn);
+            // four times the second differences of gradient2 (:346-355) applied twice
+            Second s2;
+            if (inner) {
+                const long long c2 = 2 * sSmI[a + 2][b + 2];
+                s2.xx = sSmI[a + 2][b + 4] - c2 + sSmI[a + 2][b];
+                s2.yy = sSmI[a + 4][b + 2] - c2 + sSmI[a][b + 2];
+                s2.xy = (sSmI[a + 3][b + 3] - sSmI[a + 1][b + 3]) - (sSmI[a + 3][b + 1] - sSmI[a + 1][b + 1]);
+            } else {
+                s2 = second_border(sSmI, i, j, h, w, i0, j0);
             }
+            float x, y;
+            if (sE[a + HE][b + HE] > p.thresh) {
+                const float sgn = (s2.xy < 0) ? 1.f : ((s2.xy > 0) ? -1.f : 0.f);
+                constexpr double kEps = 1e-5;
+                constexpr float kEpsHi = (float)kEps, kEpsLo = (float)(kEps - (double)kEpsHi);
+                x = df_add(df_second(s2.xx, down), make_float2(kEpsHi, kEpsLo)).x;
+                y = df_second(s2.yy, down).x * sgn;
+            } else {  // no candidate: its direction is a weight, a rounding or two of the scaling do not matter
+                const float k = down * (1.f / 2500.f);
+                x = fmaf(__ll2float_rn(s2.xx), k, 1e-5f);
+                y = __ll2float_rn(s2.xy < 0 ? s2.yy : -s2.yy) * k;
+                if (s2.xy == 0) y = 0.f;
+            }
+            const float2 d = x != 0.f ? hessian_dir(x, y) : hessian_dir0(x, y);
             sDir[a][b] = d;
             p.dir[M.px_base + (long long)i * w + j] = d;
         }
         __syncthreads();
+    } else if (df_tile) {
+        orient_df(p, M, sE, sStage, sDir, i0, j0);
     } else if (M.theta == nullptr) {
         const float tri[9] = {1.f / 25, 2.f / 25, 3.f / 25, 4.f / 25, 5.f / 25, 4.f / 25, 3.f / 25, 2.f / 25, 1.f / 25};
+#pragma unroll 1
         for (int q = tid; q < NE * (kT + 4); q += blockDim.x) {
             const int a = q / (kT + 4), c = q - a * (kT + 4);
             float acc = 0.f;
@@ -350,6 +488,7 @@ __global__ void __launch_bounds__(256, 5) tc_orient_nms(const __grid_constant__ 
             sTmp[a][c] = acc;
         }
         __syncthreads();
+#pragma unroll 1
         for (int q = tid; q < (kT + 4) * (kT + 4); q += blockDim.x) {
             const int d = q / (kT + 4), c = q - d * (kT + 4);
             float acc = 0.f;
@@ -359,6 +498,7 @@ __global__ void __launch_bounds__(256, 5) tc_orient_nms(const __grid_constant__ 
         }
         __syncthreads();
         // gradient2 (:346-355): central differences, one-sided at the borders
+#pragma unroll 1
         for (int q = tid; q < (kT + 2) * (kT + 2); q += blockDim.x) {
             const int e = q / (kT + 2), f = q - e * (kT + 2);
             const int i = i0 - 1 + e, j = j0 - 1 + f;
@@ -376,6 +516,7 @@ __global__ void __launch_bounds__(256, 5) tc_orient_nms(const __grid_constant__ 
         __syncthreads();
     }
     const float PI_F = 3.14159265358979323846f;
+#pragma unroll 1
     for (int q = tid; q < kT * kT && !df_tile; q += blockDim.x) {
         const int a = q >> 5, b = q & 31;
         const int i = i0 + a, j = j0 + b;
@@ -394,13 +535,7 @@ __global__ void __launch_bounds__(256, 5) tc_orient_nms(const __grid_constant__ 
                 const float sgn = (oxy < 0.f) ? 1.f : ((oxy > 0.f) ? -1.f : 0.f);
                 const float x = oxx + 1e-5f, y = oyy * sgn;
                 if (x != 0.f) {
-                    // th = atan(y / x) (:370-371) lies in (-pi/2, pi/2), so
-                    // wrap_mod_pi (:216-222) adds pi exactly when th < 0, and
-                    // compute_dir_from_theta (:296-305) is (cos, sin) of that:
-                    // (|x|, y sgn x) / |(x, y)|, negated when x y < 0
-                    const float rn = rsqrtf(fmaf(x, x, y * y));
-                    const float cx = fabsf(x) * rn, sy = copysignf(1.f, x) * y * rn;
-                    const float2 d = (x * y < 0.f) ? make_float2(-cx, -sy) : make_float2(cx, sy);
+                    const float2 d = hessian_dir(x, y);
                     sDir[a][b] = d;
                     p.dir[M.px_base + (long long)i * w + j] = d;
                     continue;
@@ -594,6 +729,37 @@ __global__ void __launch_bounds__(256, 5) tc_orient_nms(const __grid_constant__ 
         }
         p.eid[M.px_base + (long long)i * w + j] = id;
     }
+}
+
+// A staged edgel as tc_orient_nms leaves it: its work-grid pixel and the FP32
+// offset from it.
+struct Packed {
+    int cj, ci;
+    float ox, oy;
+};
+__device__ __forceinline__ Packed load_packed(const Scratch& sc, long long r)
+{
+    const int4 v = *reinterpret_cast<const int4*>(&sc.staging[r]);
+    return {v.y, v.w, __int_as_float(v.x), __int_as_float(v.z)};
+}
+// The position in work pixels, as the correction emits it.
+__device__ __forceinline__ double2 packed_pos(const SubParams& p, const Packed& e)
+{
+    return p.hyb ? make_double2((double)e.cj + (double)e.ox, (double)e.ci + (double)e.oy)
+                 : make_double2((double)((float)e.cj + e.ox), (double)((float)e.ci + e.oy));
+}
+// Whether two edgels lie within the radius of each other (r2 its square, in
+// original pixels): FP32 on the pixels' difference plus the offsets', FP64 as
+// the reference compares where that is closer to the radius than FP32
+// positions of a 2^16 wide grid resolve.
+__device__ __forceinline__ bool within(const SubParams& p, const SubMap& M, const Packed& a, const Packed& b, double r2)
+{
+    const float fx = (float)(a.cj - b.cj) + (a.ox - b.ox), fy = (float)(a.ci - b.ci) + (a.oy - b.oy);
+    const float d2 = fmaf(fx, fx, fy * fy), s2 = (float)r2 * (float)(M.scale * M.scale);
+    if (fabsf(d2 - s2) > 0.05f * (1.f + s2)) return d2 < s2;
+    const double2 pa = packed_pos(p, a), pb = packed_pos(p, b);
+    const double inv = 1.0 / (double)M.scale, dx = pa.x * inv - pb.x * inv, dy = pa.y * inv - pb.y * inv;
+    return dx * dx + dy * dy <= r2;
 }
 
 // ---------------------------------------------------------------------------
@@ -795,8 +961,8 @@ __global__ void __launch_bounds__(512, 2) tc_correct(const __grid_constant__ Sub
         // unpack tc_orient_nms's (pixel, FP32 offset) positions and FP32 strength
         const int cj = __double2hiint(rec.x), ci = __double2hiint(rec.y);
         const float ox = __int_as_float(__double2loint(rec.x)), oy = __int_as_float(__double2loint(rec.y));
-        const double sx = p.hyb ? (double)cj + (double)ox : (double)((float)cj + ox);
-        const double sy = p.hyb ? (double)ci + (double)oy : (double)((float)ci + oy);
+        const double2 pos = packed_pos(p, {cj, ci, ox, oy});
+        const double sx = pos.x, sy = pos.y;
         rec.w = (double)__int_as_float(__double2loint(rec.w));
         // cell and fraction of the position: from the pixel and its FP32 offset
         // (the fraction correctly rounded to FP32, as (float)(sx - floor(sx)))
@@ -941,10 +1107,24 @@ __global__ void __launch_bounds__(256) tc_isolate(const __grid_constant__ SubPar
             p.keep[r] = 1;
             continue;
         }
-        const double4_32a me = p.sc.staging[r];
-        const int pi = (int)floor(me.y * M.scale), pj = (int)floor(me.x * M.scale);
+        const Packed me = load_packed(p.sc, r);
+        const int pi = me.ci, pj = me.cj;
         bool found = false;
+        // the eight pixels around it first, all loads in flight together: a
+        // contour's next edgel is nearly always there
+        int near[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int v = u < 4 ? u : u + 1, ii = pi + v / 3 - 1, jj = pj + v % 3 - 1;
+            near[u] = (unsigned)ii < (unsigned)M.h && (unsigned)jj < (unsigned)M.w
+                          ? p.eid[M.px_base + (long long)ii * M.w + jj]
+                          : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (!found && near[u] >= 0) found = within(p, M, me, load_packed(p.sc, near[u]), r2);
         for (int d = 0; d <= reach && !found; ++d) {
+            if (d == 1) continue;  // those eight
             for (int ii = pi - d; ii <= pi + d && !found; ++ii) {
                 if (ii < 0 || ii >= M.h) continue;
                 const int step = (ii == pi - d || ii == pi + d) ? 1 : 2 * d;  // ring: full edge rows, end columns
@@ -955,9 +1135,7 @@ __global__ void __launch_bounds__(256) tc_isolate(const __grid_constant__ SubPar
                     // the reference looks only in the 3 x 3 cells of size radius
                     // around the edgel's cell; every edgel within the radius
                     // lies in one of them, so the distance test alone decides
-                    const double4_32a ot = p.sc.staging[o];
-                    const double ddx = me.x - ot.x, ddy = me.y - ot.y;
-                    if (ddx * ddx + ddy * ddy <= r2) {
+                    if (within(p, M, me, load_packed(p.sc, o), r2)) {
                         found = true;
                         break;
                     }
@@ -995,7 +1173,89 @@ __global__ void __launch_bounds__(256) tc_compact(const __grid_constant__ SubPar
     }
 }
 
-// Dense TO_E / TO_O (:708-715): pass 0 elects, per pixel, the last edgel in
+// Dense TO_E / TO_O (:708-715) at interp_n = 0, one pass: an edgel lies within
+// sqrt(2) of its pixel, so it rounds onto it or one of the eight around, and
+// the edgel that a pixel gets -- the last in list order, row-major by pixel --
+// is the last of the tile's and its neighbours' pixels, in row-major order,
+// whose edgel rounds onto it: a vote in shared memory.  Every pixel
+// is written, edgel or not: no winner map (4 bytes a pixel cleared and voted
+// on) and no cleared output.  Runs before the lists are compacted.
+__global__ void __launch_bounds__(256) tc_dense_gather(const __grid_constant__ SubParams p)
+{
+    constexpr int NH = kT + 2;
+    __shared__ int sId[NH * NH];   // edgels of the tile and one pixel around
+    __shared__ int sWin[kT * kT];  // per pixel the last of them (row-major) that rounds onto it, or -1
+    const int t = blockIdx.x;
+    const int k = find_image(p.n_maps, t, [&](int i) { return p.m[i].tile_base; });
+    const SubMap& M = p.m[k];
+    if (M.TO_E == nullptr && M.TO_O == nullptr) return;
+    const int h = M.h, w = M.w;
+    const int lt = t - M.tile_base;
+    const int ty = lt / M.ntx, tx = lt - ty * M.ntx;
+    const int i0 = ty * kT, j0 = tx * kT;
+    const int tid = threadIdx.x;
+    // segments (row, tile column) of the tile and around it: any edgels?
+    bool any = false;
+    if (tid < 3 * NH) {
+        const int i = i0 - 1 + tid / 3, c = tx - 1 + tid % 3;
+        if (i >= 0 && i < h && c >= 0 && c < M.ntx) any = p.sc.seg[M.seg_base + (long long)i * M.ntx + c].y > 0;
+    }
+    any = __syncthreads_or(any);
+    if (any) {
+        for (int q = tid; q < kT * kT; q += blockDim.x) sWin[q] = -1;
+        __syncthreads();
+        for (int a = tid >> 5; a < NH; a += 8) {  // a warp per row
+            const int i = i0 - 1 + a;
+            if ((unsigned)i >= (unsigned)h) continue;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const int b = (tid & 31) + 32 * c, j = j0 - 1 + b;
+                if (b >= NH || (unsigned)j >= (unsigned)w) continue;
+                const int id = p.eid[M.px_base + (long long)i * w + j];
+                if (id < 0 || !p.keep[id]) continue;
+                const double2 xy = *reinterpret_cast<const double2*>(&p.sc.staging[id]);
+                const int X = max(0, min((int)round(xy.x), w - 1)) - j0, Y = max(0, min((int)round(xy.y), h - 1)) - i0;
+                sId[a * NH + b] = id;
+                if ((unsigned)X < (unsigned)kT && (unsigned)Y < (unsigned)kT) atomicMax(&sWin[Y * kT + X], a * NH + b);
+            }
+        }
+        __syncthreads();
+    }
+    // four pixels of a row a thread
+    const int a = tid >> 3, b = 4 * (tid & 7), i = i0 + a, j = j0 + b;
+    if (i >= h || j >= w) return;
+    double2 ow[4];  // orientation, strength
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int win = any ? sWin[a * kT + b + u] : -1;
+        ow[u] = win >= 0 ? *(reinterpret_cast<const double2*>(&p.sc.staging[sId[win]]) + 1) : make_double2(0.0, 0.0);
+    }
+    const long long o = (long long)i * w + j;
+    const bool vec = !p.out_f64 && (w & 3) == 0 &&
+                     ((reinterpret_cast<uintptr_t>(M.TO_E) | reinterpret_cast<uintptr_t>(M.TO_O)) & 15u) == 0;
+    if (vec) {  // (w a multiple of 4, so all four are inside)
+        if (M.TO_E)
+            *reinterpret_cast<float4*>(static_cast<float*>(M.TO_E) + o) =
+                make_float4((float)ow[0].y, (float)ow[1].y, (float)ow[2].y, (float)ow[3].y);
+        if (M.TO_O)
+            *reinterpret_cast<float4*>(static_cast<float*>(M.TO_O) + o) =
+                make_float4((float)ow[0].x, (float)ow[1].x, (float)ow[2].x, (float)ow[3].x);
+        return;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        if (j + u >= w) break;
+        if (p.out_f64) {
+            if (M.TO_E) static_cast<double*>(M.TO_E)[o + u] = ow[u].y;
+            if (M.TO_O) static_cast<double*>(M.TO_O)[o + u] = ow[u].x;
+        } else {
+            if (M.TO_E) static_cast<float*>(M.TO_E)[o + u] = (float)ow[u].y;
+            if (M.TO_O) static_cast<float*>(M.TO_O)[o + u] = (float)ow[u].x;
+        }
+    }
+}
+
+// The same on a finer work grid: pass 0 elects, per pixel, the last edgel in
 // list order that rounds onto it; pass 1 writes its strength and orientation.
 template <int PASS>
 __global__ void __launch_bounds__(kSegTile) tc_dense(const __grid_constant__ SubParams p)
@@ -1171,12 +1431,16 @@ cudaError_t subpix_launch(const toed_edgemap* maps, int n, const toed_subpix_par
     if (e == cudaSuccess) e = cudaMemsetAsync(s.img_count, 0, sizeof(int) * n, stream);
     void* args[] = {p};
     if (e == cudaSuccess) e = cudaLaunchKernel((const void*)tc_orient_nms, dim3(tiles), dim3(256), args, 0, stream);
+    if (e == cudaSuccess) e = cudaLaunchKernel((const void*)tc_isolate, dim3(p->n_seg_tiles), dim3(256), args, 0, stream);
     size_t smem = 0;
     const void* cf = correct_entry(r, &smem);
     if (!cf) return cudaErrorInvalidValue;
     if (e == cudaSuccess) e = cudaFuncSetAttribute(cf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) e = cudaLaunchKernel(cf, dim3(tiles), dim3(512), args, smem, stream);
-    if (e == cudaSuccess) e = cudaLaunchKernel((const void*)tc_isolate, dim3(p->n_seg_tiles), dim3(256), args, 0, stream);
+    bool dense = false;
+    for (int i = 0; i < n; ++i) dense = dense || maps[i].TO_E || maps[i].TO_O;
+    if (dense && sc == 1 && e == cudaSuccess)
+        e = cudaLaunchKernel((const void*)tc_dense_gather, dim3(tiles), dim3(256), args, 0, stream);
     if (e == cudaSuccess) e = cudaLaunchKernel((const void*)tc_compact, dim3(p->n_seg_tiles), dim3(256), args, 0, stream);
     // ordering pass shared with the detector
     BatchParams* b = new BatchParams();
@@ -1200,9 +1464,7 @@ cudaError_t subpix_launch(const toed_edgemap* maps, int n, const toed_subpix_par
         d.W = p->m[i].w;
     }
     if (e == cudaSuccess) e = launch_finalize_subpix(*b, stream);
-    bool dense = false;
-    for (int i = 0; i < n; ++i) dense = dense || maps[i].TO_E || maps[i].TO_O;
-    if (dense && e == cudaSuccess) {
+    if (dense && sc > 1 && e == cudaSuccess) {
         e = cudaMemsetAsync(s.win, 0xff, sizeof(int) * (size_t)px, stream);
         const size_t es = p->out_f64 ? sizeof(double) : sizeof(float);
         for (int i = 0; i < n && e == cudaSuccess; ++i) {
