@@ -94,6 +94,10 @@ struct DetImage {
     int unit_base;       // first work unit
     int tile_base;       // first ordering tile
     int ed_base;         // first edgel-kernel tile
+    int band_base;       // first band (row of edgel-kernel tiles) in Scratch::band
+    void* host_out;      // mapped host memory that the list is copied to as its bands are complete, or null
+    int* host_index;
+    int* host_count;
     int tma;             // 1: rows arrive by TMA through BatchParams::tmap[k]; 0: by loads
     int wait_slot;       // 0: pixels ready at launch; g > 0: the copy engine is still bringing them in,
                          // BatchParams::ready[g - 1] reads ready_epoch once they are complete
@@ -110,6 +114,7 @@ struct Scratch {
     long long seg_cap;   // segments `seg` holds
     int* tile_sum;       // per ordering tile
     long long* img_base; // per image: exclusive prefix of its first segment
+    int* band;           // per band of an image with host_out: edgel-kernel tiles done
     int* seg_dst;        // per segment: its place in its image's list
     unsigned long long* tile_state;  // per scan tile: {0, 1 its count, 2 the count of its image's
                                      // tiles up to it} << 32 | count
@@ -163,6 +168,7 @@ struct BatchParams {
     int seg_tile;        // segments per ordering tile: kSegTile, or kScanTileMax
     int ed_rows;         // image rows of an edgel-kernel tile (one strip column wide), up to kEdRowsMax
     int n_ed;            // such tiles
+    int n_bands;         // bands to count (0: no list goes to host memory)
     int hyb;             // 1: peak fit on exact FP32 differences, FP64 recomputation of ill-conditioned
                          // orientations (TOED_HYBRID)
     int qad;             // 1: orientation from derivatives interpolated at the subpixel point (TOED_ORI_QAD)

@@ -424,6 +424,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<R, NMSTO>::MINB)
     // the scan, which runs after this kernel, takes tiles by a ticket and
     // publishes tile states: both start at zero
     for (int i = blockIdx.x * kThreads + tid; i < p.n_tiles; i += gridDim.x * kThreads) p.sc.tile_state[i] = 0ull;
+    for (int i = blockIdx.x * kThreads + tid; i < p.n_bands; i += gridDim.x * kThreads) p.sc.band[i] = 0;
     if (blockIdx.x == 0 && tid == 0) p.sc.words[3] = 0;
     int stg_next = 0, stg_end = 0;  // this warp's reserved staging range [next, end) (uniform)
     if (tid == 0) {

@@ -114,6 +114,7 @@ __global__ void __launch_bounds__(kScanThreads) fin_scan(const __grid_constant__
             s_scal[1] = excl;
             if (t + 1 == (k + 1 < p.n_img ? p.img[k + 1].tile_base : p.n_tiles)) {  // the image's last tile
                 *im.count = excl + total;
+                if (im.host_count) *im.host_count = excl + total;
                 if (excl + total > im.cap) atomicOr(&p.sc.words[2], TOED_FLAG_OVER_CAPACITY);
             }
         }

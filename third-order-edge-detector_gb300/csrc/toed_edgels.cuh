@@ -402,6 +402,34 @@ __device__ __forceinline__ Subpixel subpixel_of(const Staged& e, int W2, bool hy
     return {px - fx, py - fy, min(max((int)fx, Gc - 2), Gc + 1), min(max((int)fy, Gr - 2), Gr + 1)};
 }
 
+// A tile of band `ty` is done: the CTA that completes the band -- tiles of all
+// strip columns over the same rows, whose edgels are consecutive in the list --
+// copies its part of the list to the host, in whole lines.  So the lists cross
+// the link while later bands are worked on.  (The tiles' own stores, single
+// records at scattered places, took 0.45 ms more per 40 MB over the link; a copy
+// kernel afterwards 0.2 ms.)
+static __device__ __noinline__ void band_done(const BatchParams& p, const DetImage& im, int ty, int* s_last)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        *s_last = atomicAdd(&p.sc.band[im.band_base + ty], 1) == im.nsc - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!*s_last) return;
+    const long long row = 2LL * p.ed_rows * im.nsc;  // segments a band
+    const long long q0 = ty * row, q1 = q0 + row;
+    const int lo = min(p.sc.seg_dst[im.seg_base + q0], im.cap);
+    const int hi = min(q1 < im.nseg ? p.sc.seg_dst[im.seg_base + q1] : *im.count, im.cap);
+    const int per = p.out_f64 ? 2 : 1;  // 16-byte parts of a record
+    const uint4* src = static_cast<const uint4*>(im.out);
+    uint4* dst = static_cast<uint4*>(im.host_out);
+    for (long long i = (long long)lo * per + threadIdx.x; i < (long long)hi * per; i += blockDim.x) dst[i] = __ldcg(src + i);
+    if (im.host_index)
+        for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) im.host_index[i] = __ldcg(im.index + i);
+}
+
 template <int R, bool QAD>
 __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels(const __grid_constant__ BatchParams p)
 {
@@ -452,7 +480,10 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
     }
     int total;
     int run = block_excl_scan<kEdThreads>(sum, s_warp, &total);
-    if (total == 0) return;
+    if (total == 0) {
+        if (im.host_out) band_done(p, im, ty, s_warp);
+        return;
+    }
     // pixels x0 - HALO .. x0 + 29 + HALO, rows y0 - HALO .., zero outside the image, by TMA where the detection kernel's rows came so
     const int px = sc * kInner - E::HALO, py = y0 - E::HALO;
     const int x_al = floor4(px), shift = px - x_al;
@@ -615,6 +646,7 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
         }
         __syncthreads();  // the next chunk overwrites the lists
     }
+    if (im.host_out) band_done(p, im, ty, s_warp);
 }
 
 struct EdEntry {

@@ -1,7 +1,6 @@
 // toed_finalize.cu -- ordering pass of the TO correction: turns staged edgels
 // and the row-segment table into each map's edgel list in row-major order
-// (the detection's lists are ordered by toed_edgels.cu); and the copy of
-// finished lists to mapped host memory.
+// (the detection's lists are ordered by toed_edgels.cu).
 //
 // Segments are (row, strip column) pairs laid out row-major per image and
 // padded to whole tiles of kSegTile.  Three short kernels:
@@ -12,8 +11,6 @@
 //                   staged records cooperatively to their list positions
 //                   (global prefix - image base), converting to the output
 //                   dtype (the quick-and-dirty mode: toed_qad.cu).
-#include <algorithm>
-
 #include "toed_common.cuh"
 #include "toed_internal.h"
 
@@ -113,49 +110,6 @@ __global__ void __launch_bounds__(kFinThreads) fin_scatter(const __grid_constant
             reinterpret_cast<float4*>(im.out)[d] = make_float4((float)rc.x, (float)rc.y, (float)rc.z, (float)rc.w);
         }
     }
-}
-
-// Lists to mapped host memory: whole lines written by consecutive threads.
-// (The edgel kernel's own stores are single records at scattered places: over
-// the link they took 0.45 ms more per 40 MB of lists.)
-struct ListCopies {
-    ListCopy l[kBatchMax];
-    int rec;
-};
-
-__global__ void __launch_bounds__(256) fin_list_copy(const __grid_constant__ ListCopies p)
-{
-    const ListCopy& l = p.l[blockIdx.y];
-    const int cnt = *l.count, n = min(cnt, l.cap);
-    const long long nv = (long long)n * p.rec / 16;
-    const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, st = (long long)gridDim.x * blockDim.x;
-    const uint4* src = static_cast<const uint4*>(l.src);
-    uint4* dst = static_cast<uint4*>(l.dst);
-    for (long long i = t0; i < nv; i += st) dst[i] = src[i];
-    if (l.idx)
-        for (long long i = t0; i < n; i += st) l.idx_dst[i] = l.idx[i];
-    if (t0 == 0) *l.count_dst = cnt;
-}
-
-cudaError_t preload_list_copy()
-{
-    cudaFuncAttributes fa;
-    return cudaFuncGetAttributes(&fa, (const void*)fin_list_copy);
-}
-
-cudaError_t launch_list_copy(const ListCopy* lists, int n, int rec, cudaStream_t stream)
-{
-    for (int i0 = 0; i0 < n; i0 += kBatchMax) {
-        ListCopies p;
-        const int m = n - i0 < kBatchMax ? n - i0 : kBatchMax;
-        for (int i = 0; i < m; ++i) p.l[i] = lists[i0 + i];
-        p.rec = rec;
-        void* args[] = {&p};
-        // enough stores in flight to fill the link whatever the number of lists
-        const cudaError_t e = cudaLaunchKernel((const void*)fin_list_copy, dim3(std::max(8, 1024 / m), m), dim3(256), args, 0, stream);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
 }
 
 cudaError_t launch_finalize_subpix(const BatchParams& p, cudaStream_t stream)

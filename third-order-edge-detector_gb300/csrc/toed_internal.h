@@ -24,21 +24,6 @@ cudaError_t launch_finalize_subpix(const BatchParams& p, cudaStream_t stream);
 cudaError_t prepare_edgels(int radius, bool qad);  // the edgel kernel's attributes, once per device, radius and mode
 cudaError_t prepare_qad(int radius);
 cudaError_t launch_qad(const BatchParams& p, cudaStream_t stream);
-
-// One finished list from device memory to its mapped host buffers
-// (toed_finalize.cu): min(count, cap) records of `rec` bytes, the grid
-// indices where wanted, and the count.
-struct ListCopy {
-    const void* src;
-    void* dst;
-    const int* idx;
-    int* idx_dst;
-    const int* count;
-    int* count_dst;
-    int cap;
-};
-cudaError_t launch_list_copy(const ListCopy* lists, int n, int rec, cudaStream_t stream);
-cudaError_t preload_list_copy();
 // Load those kernels for `radius` (and the QaD variant) now:
 // with lazy module loading a kernel's first launch may wait for the device,
 // which must not happen while a detection launch waits for copies that the
