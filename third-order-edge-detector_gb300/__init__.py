@@ -480,20 +480,19 @@ class Detector:
         """Adjoint of detect_batch with the selection frozen: given the
         forward's images, its per-image grid indices and dL/d(edgels)
         (N x 4 each), returns (dL/dimages as float32 tensors, dL/dsigma)."""
-        grads, gs, _ = self._adjoint(images, indices, grad_edgels, sigma, radius, out_dtype, stream)
-        return grads, gs
-
-    def _adjoint(self, images, indices, grad_edgels, sigma, radius, out_dtype=TOED_F32, stream=None):
-        """backward_batch; the third value is the (n, H, W) buffer that images
-        of one size share for their gradients, or None."""
         t = self.torch
         dev = t.device("cuda", self.device)
-        items, grads = [], []
+        grads = [t.empty(im.shape, dtype=t.float32, device=dev) for im in images]
+        return grads, self._adjoint(images, indices, grad_edgels, grads, sigma, radius, out_dtype, stream)
+
+    def _adjoint(self, images, indices, grad_edgels, grads, sigma, radius, out_dtype=TOED_F32, stream=None):
+        """backward_batch into the given contiguous gradients; dL/dsigma."""
+        t = self.torch
+        dev = t.device("cuda", self.device)
+        items = []
         gdt = t.float64 if out_dtype == TOED_F64 else t.float32
         keep = []
-        same = len(images) > 0 and all(im.shape == images[0].shape for im in images)
-        flat = t.empty((len(images), *images[0].shape), dtype=t.float32, device=dev) if same else None
-        for k, (im, idx, ge) in enumerate(zip(images, indices, grad_edgels)):
+        for im, idx, ge, gp in zip(images, indices, grad_edgels, grads):
             if im.stride(1) != 1:
                 raise ValueError("image rows must be contiguous")
             H, W = im.shape
@@ -501,9 +500,7 @@ class Detector:
                 idx.to(device=dev, dtype=t.int32).contiguous()
             go = ge if ge.dtype == gdt and ge.device == dev and ge.is_contiguous() else \
                 ge.to(device=dev, dtype=gdt).contiguous()
-            gp = flat[k] if same else t.empty((H, W), dtype=t.float32, device=dev)
             keep += [gi, go]
-            grads.append(gp)
             items.append(toed_grad_image(im.data_ptr(), H, W, im.stride(0),
                                          TOED_U8 if im.dtype == t.uint8 else TOED_F32, int(gi.numel()),
                                          gi.data_ptr() if gi.numel() else None,
@@ -514,7 +511,7 @@ class Detector:
         s = stream if stream is not None else t.cuda.current_stream(self.device)
         _check(lib().toed_backward_batch(self._ctx, arr, len(items), ctypes.byref(p), ctypes.c_void_p(gs.data_ptr()),
                                          ctypes.c_void_p(s.cuda_stream)), "toed_backward_batch")
-        return grads, gs, flat
+        return gs
 
     def subpix_to_correct_batch(self, maps, thresh=0.2, sigma=2.0, nbr_radius=2.0, thetas=None,
                                 out_dtype=TOED_F32, precision=TOED_HYBRID, capacity=None, dense=True,
@@ -742,7 +739,8 @@ def differentiable_detect(images, sigma, threshold=2.0, radius=0, detector=None)
         def backward(ctx, g_edg, g_idx, g_cnt):
             (imgs,) = ctx.saved_tensors
             splits = torch.split(g_edg.contiguous(), ctx.counts)
-            _, gs, flat = det._adjoint(list(imgs), ctx.idx, list(splits), ctx.sigma, radius)
+            flat = torch.empty(imgs.shape, dtype=torch.float32, device=torch.device("cuda", det.device))
+            gs = det._adjoint(list(imgs), ctx.idx, list(splits), list(flat.unbind(0)), ctx.sigma, radius)
             gi = flat if ctx.needs_input_grad[0] else None
             gsig = gs.reshape(()).to(dtype=ctx.sig_meta[0], device=ctx.sig_meta[1]) if ctx.needs_input_grad[1] else None
             return gi, gsig

@@ -1175,9 +1175,9 @@ extern "C" toed_status toed_backward_batch(toed_ctx* c, const toed_grad_image* i
     toed_status st = TOED_OK;
     {
         std::lock_guard<std::mutex> lk(c->mu);
-        cudaError_t e = cudaMemsetAsync(grad_sigma, 0, sizeof(double), stream);
+        cudaError_t e = cudaSuccess;
         for (int i0 = 0; i0 < n && e == cudaSuccess; i0 += kBatchMax)
-            e = backward_launch(items + i0, std::min(kBatchMax, n - i0), prm, r, grad_sigma, stream);
+            e = backward_launch(items + i0, std::min(kBatchMax, n - i0), prm, r, grad_sigma, i0 == 0, stream);
         if (e != cudaSuccess) {
             g_last_cuda_error = std::string("backward: ") + cudaGetErrorString(e);
             st = TOED_ERR_CUDA;

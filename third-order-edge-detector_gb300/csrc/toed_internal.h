@@ -46,8 +46,8 @@ toed_status check_image(const toed_image& im);
 void encode_rows_map(CUtensorMap* m, DetImage& d, int radius);
 
 // Enqueue the adjoint (toed_backward.cu): clears each item's grad_pixels,
-// then one kernel; dL/dsigma is added into *gsig.
-cudaError_t backward_launch(const toed_grad_image* items, int n, const toed_params* prm, int r, double* gsig,
+// and, if first, *gsig, then one kernel; dL/dsigma is added into *gsig.
+cudaError_t backward_launch(const toed_grad_image* items, int n, const toed_params* prm, int r, double* gsig, bool first,
                             cudaStream_t stream);
 
 // Scratch of the TO-correction pipeline (owned by the caller's context).
