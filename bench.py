@@ -4,7 +4,7 @@ Workload (the metric's batched configuration): 64 seeded synthetic float32
 images, width and height each U[256, 2048] rounded to multiples of 4
 (79.4 Mpixel in total), shapes generator with noise std U[1, 8], sigma 1.5
 (r = 6), threshold 2.0, one persistent launch per step.  A step is one
-detection pass over the whole batch (detection kernel + ordering pass).
+detection pass over the whole batch (detection, scan and edgel kernels).
 
 * ``value``   : Mpixel/s with the images already resident in HBM (CUDA events
                 on the launching stream, max over ranks).  Inputs (318 MB) are
@@ -429,7 +429,7 @@ def side_measurements(toed, det, images, side, stream):
     for sg in (1.0, 2.0):
         p1 = toed.make_params(sg)
         det.autotune([c1], o1, p1, reps=5)  # this size class's launch shape
-        # as deployed: the detection and the ordering pass replayed from a CUDA graph ...
+        # as deployed: detection, scan and edgel kernels replayed from a CUDA graph ...
         g1 = det.capture([c1], o1, p1)
         ms = _time_ms(lambda: g1.replay(), 50, stream)
         out[f"single_752x480_u8_sigma{sg:g}_mpx_s"] = round(c1.numel() / (ms * 1e-3) / 1e6, 1)
@@ -766,12 +766,12 @@ def run_ours(args, ws, rank, local):
         "vs_baseline": None, "dtype": "f32 (peak fit on exact FP32 differences; FP64 TO orientation where the vector cancels)",
         "data": "synthetic (seeded shapes generator; inputs 318 MB > L2, no flush needed)",
         "config": {"workload": "uneven batch: 64 float32 images, H and W U[256,2048] (x4), noise U[1,8]",
-                   "launch": "one CUDA graph per step (persistent detection kernel + 3-kernel ordering pass)",
+                   "launch": "one CUDA graph per step (persistent detection kernel, scan, edgel kernel)",
                    "autotuned": {"strip_rows": tuned["strip_rows"], "staging": tuned["staging"]},
                    "pixels_per_gpu": npx, "images_per_gpu": len(images), "sigma": SIGMA, "radius": r,
                    "threshold": THRESH, "edgels_per_gpu": n_edgels, "parallelism": f"replicas x{ws}",
                    "l2": "inputs larger than L2"},
-        "gpu_launches": 4 * args.steps,
+        "gpu_launches": 3 * args.steps,
         "kernel_ms": round(kernel_ms, 4),
         "e2e": {"value": round(ws * npx / (e2e_ms * 1e-3) / 1e6, 2), "unit": "Mpixel/s",
                 "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h_total),
