@@ -1095,7 +1095,7 @@ __global__ void __launch_bounds__(256) tc_isolate(const __grid_constant__ SubPar
     // an edgel lies within sqrt(2) work pixels of its own; search the id map
     // (work grid) around it, compare in original pixels as the reference does
     const int reach = (int)ceil(p.nbr * M.scale + 1.5);
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
+    for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < total; e += gridDim.y * blockDim.x) {
         int lo = 0, hi = kSegTile - 1;  // last segment with s_dst <= e
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -1462,7 +1462,12 @@ cudaError_t subpix_launch(const toed_edgemap* maps, int n, const toed_subpix_par
     if (e == cudaSuccess) e = cudaMemsetAsync(s.img_count, 0, sizeof(int) * n, stream);
     void* args[] = {p};
     if (e == cudaSuccess) e = cudaLaunchKernel((const void*)tc_orient_nms, dim3(tiles), dim3(256), args, 0, stream);
-    if (e == cudaSuccess) e = cudaLaunchKernel((const void*)tc_isolate, dim3(p->n_seg_tiles), dim3(256), args, 0, stream);
+    // few tiles of segments are shared out, each over several CTAs, until some four
+    // CTAs an SM have work: the FP64 distance tests of 22 tiles (two 501 x 667
+    // work grids) kept 22 SMs busy, 107 us against 45 shared out eight ways.  From
+    // 305 tiles on a CTA takes a whole one (1024 tiles: 110 us)
+    const unsigned shares = (unsigned)std::min(8, std::max(1, 608 / p->n_seg_tiles));
+    if (e == cudaSuccess) e = cudaLaunchKernel((const void*)tc_isolate, dim3(p->n_seg_tiles, shares), dim3(256), args, 0, stream);
     size_t smem = 0;
     const void* cf = correct_entry(r, &smem);
     if (!cf) return cudaErrorInvalidValue;
