@@ -81,12 +81,13 @@ def test_8bit_rows_from_any_alignment(toed, synth, shape, start):
     assert a["count"] == b["count"] > 0 and torch.equal(a["edgels"], b["edgels"]) and torch.equal(a["index"], b["index"])
 
 
-def test_isolation_tiles_shared_out_or_whole(detector, synth, toed):
-    """A map's segment tiles are shared out over CTAs alone, taken whole among ten maps (320 tiles)."""
-    E = [torch.as_tensor(synth.ridge_map(1024, 1024, seed=66 + k, n_curves=9).astype(np.float32)).cuda() for k in range(10)]
-    together = detector.subpix_to_correct_batch(E, thresh=0.1, sigma=1.0, nbr_radius=2.0)
+@pytest.mark.parametrize("side,interp_n", [(1024, 0), (512, 1)])
+def test_segment_tiles_shared_out_or_whole(detector, synth, toed, side, interp_n):
+    """A map's segment tiles (isolation; dense maps of a work grid) are shared out over CTAs alone, taken whole among ten maps (320 tiles)."""
+    E = [torch.as_tensor(synth.ridge_map(side, side, seed=66 + k, n_curves=9).astype(np.float32)).cuda() for k in range(10)]
+    together = detector.subpix_to_correct_batch(E, thresh=0.1, sigma=1.0, nbr_radius=2.0, interp_n=interp_n)
     for k in (0, 9):
-        alone = detector.subpix_to_correct_batch([E[k]], thresh=0.1, sigma=1.0, nbr_radius=2.0)[0]
+        alone = detector.subpix_to_correct_batch([E[k]], thresh=0.1, sigma=1.0, nbr_radius=2.0, interp_n=interp_n)[0]
         assert alone["count"] == together[k]["count"] > 100
         for name in ("edgels", "TO_E", "TO_O"):
             assert torch.equal(alone[name], together[k][name])
