@@ -428,8 +428,8 @@ __device__ __noinline__ int eval_edgel_warp(const BwImage& im, int rho, int kap,
 // latter); a third-order vector below kIllVector of its terms' magnitudes.  With
 // these limits the gradients of 72 noisy images (777 x 1001, sigma 2) differ by
 // up to 1e-6 of their norm from those all summed in the fixed order, without
-// them by up to 1.4e-4, one edgel in fifty pays (20 of 220 us; half of the faint
-// edgels, 180 us, without kIllCurve).  An edgel whose cotangents are all zero is
+// them by up to 1.4e-4; few edgels pay (6 of 219 us; with every faint edgel's
+// cotangents used, 243 us, but 388 without kIllCurve).  An edgel whose cotangents are all zero is
 // not used: zero times a finite gradient.
 constexpr float kIllStrength = 3e-4f, kIllFit = 1e-3f, kIllCurve = 0.12f, kIllVector = 0.25f;
 
@@ -796,7 +796,9 @@ __global__ void __launch_bounds__(kBwAdjThreads, BwCfg<R>::MINB) bw_adjoint(cons
                 for (int q = 0; q < 4; ++q) go[q] = g[q];
             }
             const bool used = go[0] != 0.f || go[1] != 0.f || go[2] != 0.f || go[3] != 0.f;
-            for (unsigned ill = __ballot_sync(0xffffffffu, lane < nw && (by_warp || ill_conditioned(o, nv, xmaj, used, p.ill_curve))); ill; ill &= ill - 1) {
+            unsigned ill = __ballot_sync(0xffffffffu,
+                                         lane < nw && (by_warp || ill_conditioned(o, nv, xmaj, used, p.ill_curve)));
+            for (; ill; ill &= ill - 1) {
                 const int w = __ffs(ill) - 1;
                 const int bits = eval_edgel_warp<R>(im, __shfl_sync(0xffffffffu, rho, w), __shfl_sync(0xffffffffu, kap, w),
                                                     lane, lo, hi, rows);
