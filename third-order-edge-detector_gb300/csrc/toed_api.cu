@@ -330,6 +330,19 @@ static toed_status ensure_scratch(toed_ctx* c, long long staging, long long segs
     return TOED_OK;
 }
 
+// Staging records that `edgels` survivors of `warps` warps can take.  A warp
+// reserves a block of kStageBlk and carves requests of at most an eighth of it
+// off (larger ones are reserved by themselves), so when one no longer fits it
+// leaves less than an eighth of the block behind -- and of its last block, up
+// to all of it.
+static long long staging_records(long long edgels, long long warps)
+{
+    constexpr long long kept = kStageBlk - (kStageBlk / 8 - 1);
+    return (edgels * kStageBlk + kept - 1) / kept + warps * kStageBlk;
+}
+// Warps of a detection launch at most: 2048 threads an SM.
+static long long most_warps(const toed_ctx* c) { return 64LL * c->num_sms; }
+
 extern "C" toed_status toed_reserve(toed_ctx* c, long long max_pixels, long long max_edgels, int max_images)
 {
     if (!c || max_pixels < 0 || max_edgels < 0 || max_images < 0) return TOED_ERR_INVALID_ARG;
@@ -341,9 +354,7 @@ extern "C" toed_status toed_reserve(toed_ctx* c, long long max_pixels, long long
     const long long segs = max_pixels / 15 + 2LL * 4096 + (long long)imgs * kScanTileMax;
     const long long tiles = segs / kSegTile + imgs + 1;
     std::lock_guard<std::mutex> lk(c->mu);
-    // staging slack: one reservation block per resident warp (at most 4 CTAs per SM)
-    const long long slack = 4LL * c->num_sms * (kThreads / 32) * kStageBlk;
-    toed_status st = ensure_scratch(c, std::max(max_edgels, 1LL) + slack, segs, tiles, imgs, nullptr);
+    toed_status st = ensure_scratch(c, staging_records(max_edgels, most_warps(c)), segs, tiles, imgs, nullptr);
     cudaSetDevice(prev);
     return st;
 }
@@ -529,10 +540,9 @@ static toed_status detect_chunk(toed_ctx* c, const toed_image* images, int n, co
     p->n_ed = (int)ed;
     p->n_units = (int)units;
     p->n_tiles = (int)tiles;
-    // every resident warp may leave up to one reservation block of staging unused
     p->stage_blk = kStageBlk;
-    staging += resident * (kThreads / 32) * kStageBlk;
-    toed_status st = ensure_scratch(c, std::max(staging, 1LL), tiles * seg_tile, tiles, n, stream);
+    const long long records = staging_records(staging, resident * (kThreads / 32));
+    toed_status st = ensure_scratch(c, records, tiles * seg_tile, tiles, n, stream);
     if (st != TOED_OK) return st;
     p->sc.words = c->words;
     p->sc.staging = c->staging;
@@ -954,8 +964,7 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
                 bands += images[i].height;
                 cap += images[i].capacity;
             }
-            const long long slack = 4LL * c->num_sms * (kThreads / 32) * kStageBlk;
-            st = ensure_scratch(c, std::max(cap, 1LL) + slack, segs, segs / kSegTile, n, stream);
+            st = ensure_scratch(c, staging_records(cap, most_warps(c)), segs, segs / kSegTile, n, stream);
             if (st == TOED_OK && direct) st = grow(&c->band, &c->band_cap, bands, stream);
         }
         const HostList* hl = direct ? lists.data() : nullptr;

@@ -633,7 +633,8 @@ __global__ void __launch_bounds__(kThreads, Cfg<R, NMSTO>::MINB)
                 // staging slots for n edgels: carved from the warp's reserved
                 // range, refilled from the global cursor; more than an eighth
                 // of a reservation block at once is reserved by itself, so that
-                // little of a block is ever left behind
+                // less than an eighth of a block is left behind when it is
+                // (the staging area has room for that: staging_records)
                 auto reserve = [&](int n) {
                     int base = stg_next;
                     if (stg_next + n <= stg_end) {
