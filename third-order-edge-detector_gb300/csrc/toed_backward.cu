@@ -39,6 +39,7 @@
 #include <memory>
 
 #include "toed_common.cuh"
+#include "toed_groups.h"
 #include "toed_internal.h"
 
 namespace toed {
@@ -665,18 +666,19 @@ __global__ void __launch_bounds__(kBwAdjThreads, BwCfg<R>::MINB) bw_adjoint(cons
             // Eight lanes copy a window's row, an aligned group of four pixels
             // (16 bytes of a float image, 4 of an 8-bit one) each, a row ahead of
             // its use.  A group is copied if it holds a pixel of the row and lies
-            // (but for its ends) between the image's first and last pixel; where
-            // a window reaches outside the image, what is read there is masked to
-            // zero.
+            // wholly between the image's first and last pixel (toed_groups.h);
+            // where a window reaches outside the image, what is read there is
+            // masked to zero.
             const bool u8 = im.dtype == TOED_U8;
             const long long span = (long long)(im.H - 1) * im.pitch + im.W;
             // A round this short is cheaper a warp per edgel (below), which also
-            // takes images whose offsets need 64 bits
-            const bool by_warp = few || span + 32LL * im.pitch >= (1LL << 30);
+            // takes images whose offsets need 64 bits, and those narrower than a group
+            const bool by_warp = few || span + 32LL * im.pitch >= (1LL << 30) || im.W < 4;
             const bool inside = __all_sync(0xffffffffu, wy >= 0 && wy + NU <= im.H && wx >= 0 && wx + NU <= im.W);
             const uintptr_t src = reinterpret_cast<uintptr_t>(im.src);
             const int skew = (int)(u8 ? src & 3 : src >> 2 & 3);  // the first pixel's place in its group
             const uintptr_t first_group = src - (u8 ? skew : 4 * skew);
+            const unsigned whole = whole_groups(span);
             // the window's first pixel, from first_group
             const int own = by_warp ? 0 : (int)(wy * im.pitch) + wx + skew;
             int off[8];
@@ -685,10 +687,7 @@ __global__ void __launch_bounds__(kBwAdjThreads, BwCfg<R>::MINB) bw_adjoint(cons
             auto stage = [&](int u, int buf) {  // window row u of all windows
                 const int up = u * (int)im.pitch;
                 const uint32_t d = smem_addr(rows + buf * 32 * C::ROW);
-                auto wanted = [&](int at) {
-                    const bool of_row = NU % 4 == 1 ? (lane & 7) < C::CH : 4 * (lane & 7) - (at & 3) < NU;
-                    return of_row && (unsigned)((at | 3) - skew) < (unsigned)span + 3u;
-                };
+                auto wanted = [&](int at) { return group_copied<NU, C::CH>(at, lane & 7, skew, whole); };
                 if (u8) {
                     const uint32_t dst = d + (lane >> 3) * C::ROW + 4 * (lane & 7);
 #pragma unroll
@@ -796,8 +795,9 @@ __global__ void __launch_bounds__(kBwAdjThreads, BwCfg<R>::MINB) bw_adjoint(cons
                 for (int q = 0; q < 4; ++q) go[q] = g[q];
             }
             const bool used = go[0] != 0.f || go[1] != 0.f || go[2] != 0.f || go[3] != 0.f;
-            unsigned ill = __ballot_sync(0xffffffffu,
-                                         lane < nw && (by_warp || ill_conditioned(o, nv, xmaj, used, p.ill_curve)));
+            // (pixel by pixel too: windows over a group that is not copied)
+            unsigned ill = __ballot_sync(0xffffffffu, lane < nw && (by_warp || window_cut(wy, wx, NU, im.H, im.W, skew, span) ||
+                                                                    ill_conditioned(o, nv, xmaj, used, p.ill_curve)));
             for (; ill; ill &= ill - 1) {
                 const int w = __ffs(ill) - 1;
                 const int bits = eval_edgel_warp<R>(im, __shfl_sync(0xffffffffu, rho, w), __shfl_sync(0xffffffffu, kap, w),
