@@ -1,0 +1,33 @@
+"""Rules of the kernels' sources that no run can show: a wait that gives up
+happens on no healthy GPU."""
+import glob
+import os
+import re
+
+from conftest import PKG_DIR
+
+
+def _kernels():
+    """{name: body} of the __global__ functions."""
+    out = {}
+    for path in sorted(glob.glob(os.path.join(PKG_DIR, "csrc", "*.cu*"))):
+        src = open(path).read()
+        for m in re.finditer(r"__global__[^;{]*?\b(\w+)\(const __grid_constant__ \w+ \w+\)\s*\{", src):
+            depth, i = 1, m.end()
+            while depth:
+                depth += {"{": 1, "}": -1}.get(src[i], 0)
+                i += 1
+            out[m.group(1)] = src[m.end():i]
+    return out
+
+
+def test_no_copy_outlives_its_block():
+    """A kernel whose wait for a TMA copy gave up waits again, bounded, for what
+    is still in flight before it ends, and requests no more copies."""
+    kernels = {k: b for k, b in _kernels().items() if "mbar_wait" in b}
+    assert set(kernels) == {"toed_detect_kernel", "fin_edgels"}
+    for name, body in kernels.items():
+        gave_up = re.search(r"(\w+) = (?:32|!mbar_wait)", body).group(1)
+        last = body[body.rindex("mbar_wait") - 400:]
+        assert re.search(rf"if \({gave_up} && tid == 0\)", last), name
+    assert re.search(r"issued < min\(nbox, upto\) && !dead", kernels["toed_detect_kernel"])

@@ -434,7 +434,9 @@ __global__ void __launch_bounds__(kThreads, Cfg<R, NMSTO>::MINB)
     __syncthreads();
     int bi = 0;             // buffer of the next box to arrive by TMA
     uint32_t phase = 0;     // its mbarrier's phase
-    bool dead = false;      // a wait for a box gave up
+    // not 0 once a wait for a box gave up: 32, the box's phase (bit 0), buffer
+    // (bits 1, 2) and, in thread 0, the boxes then in flight (bits 3, 4)
+    int dead = 0;
     int slot = 0;           // of sScal that holds the unit
 
     for (;;) {
@@ -491,7 +493,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<R, NMSTO>::MINB)
         const int shift = tma ? xin - x_al : C::OFF;               // where the window starts in a staged row
         int issued = 0, ib = bi;  // thread 0: boxes requested, the next one's buffer
         auto issue = [&](int upto) {
-            for (; issued < min(nbox, upto); ++issued) {
+            for (; issued < min(nbox, upto) && !dead; ++issued) {
                 tma_load_rows(&p.tmap[k], smem_addr(sRaw + ib * (B * C::BW)), bar + 8 * ib, x_al, row0(issued),
                               (uint32_t)C::box_bytes);
                 ib = ib + 1 == C::NBUF ? 0 : ib + 1;
@@ -537,7 +539,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<R, NMSTO>::MINB)
                 float* box = sRaw + bi * (B * C::BW);
                 if (tma) {
                     if (!dead && !mbar_wait(bar + 8 * bi, phase)) {
-                        dead = true;
+                        dead = 32 | ((issued - q) & 3) << 3 | bi << 1 | (int)phase;
                         atomicOr(&p.sc.words[2], TOED_FLAG_TIMEOUT);
                     }
                 } else {
@@ -718,8 +720,16 @@ __global__ void __launch_bounds__(kThreads, Cfg<R, NMSTO>::MINB)
             rb = ring_wrap<C::RING>(rb + B);
         }
     }
-    if (dead)  // nothing may be in flight towards an exited CTA's memory
-        for (int q = 0; q < C::NBUF; ++q) mbar_wait(bar + 8 * q, phase);
+    // nothing may be in flight towards an exited CTA's memory: the boxes that
+    // thread 0 had requested when its wait gave up (it requests none after that)
+    if (dead && tid == 0)
+        for (int k = 0, q = (dead >> 1) & 3, ph = dead & 1; k < ((dead >> 3) & 3); ++k) {
+            mbar_wait(bar + 8 * q, ph);
+            if (++q == C::NBUF) {
+                q = 0;
+                ph ^= 1;
+            }
+        }
 }
 
 }  // namespace toed
