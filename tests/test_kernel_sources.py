@@ -31,3 +31,18 @@ def test_no_copy_outlives_its_block():
         last = body[body.rindex("mbar_wait") - 400:]
         assert re.search(rf"if \({gave_up} && tid == 0\)", last), name
     assert re.search(r"issued < min\(nbox, upto\) && !dead", kernels["toed_detect_kernel"])
+
+
+def test_scan_and_edgel_kernel_are_guarded():
+    """The bounds-checked build covers every kernel of a detection: the indices
+    that data decides -- segments, staged pixels and windows, records, list
+    positions, bands -- go through TOED_IN_BOUNDS."""
+    kernels = _kernels()
+    for name, least in (("toed_detect_kernel", 5), ("fin_scan", 3), ("fin_edgels", 9)):
+        assert kernels[name].count("TOED_IN_BOUNDS") >= least, name
+    src = open(os.path.join(PKG_DIR, "csrc", "toed_edgels.cuh")).read()
+    band = src[src.index("void band_done("):src.index("template <int R, bool QAD>\n__global__")]
+    assert band.count("TOED_IN_BOUNDS") >= 3
+    # every window handed to a sum is checked against the staged pixels
+    body = kernels["fin_edgels"]
+    assert len(re.findall(r"const float\* win = ", body)) == body.count("TOED_IN_BOUNDS(staged(win")

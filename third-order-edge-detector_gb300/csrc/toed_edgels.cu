@@ -93,6 +93,7 @@ __global__ void __launch_bounds__(kScanThreads) fin_scan(const __grid_constant__
     if (tid == 0) s_scal[0] = atomicAdd(&p.sc.words[3], 1);
     __syncthreads();
     const int t = s_scal[0];
+    if (!TOED_IN_BOUNDS(t < p.n_tiles, p.sc.words)) return;
     const int k = find_image(p.n_img, t, [&](int i) { return p.img[i].tile_base; });
     const DetImage& im = p.img[k];
     // (an image's segments are padded to whole tiles, so whole groups are read and written)
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(kScanThreads) fin_scan(const __grid_constant__
     int cnt[PER], sum = 0;
 #pragma unroll
     for (int u = 0; u < PER; u += 2) {
-        const int4 sg = u < left ? seg[u / 2] : make_int4(0, 0, 0, 0);
+        const int4 sg = u < left && TOED_IN_BOUNDS(im.seg_base + q0 + u + 2 <= p.sc.seg_cap, p.sc.words) ? seg[u / 2] : make_int4(0, 0, 0, 0);
         cnt[u] = sg.y;
         cnt[u + 1] = u + 1 < left ? sg.w : 0;
         sum += cnt[u] + cnt[u + 1];
@@ -130,7 +131,7 @@ __global__ void __launch_bounds__(kScanThreads) fin_scan(const __grid_constant__
         d.z = d.y + cnt[u + 1];
         d.w = d.z + cnt[u + 2];
         run = d.w + cnt[u + 3];
-        if (u < left) dst[u / 4] = d;
+        if (u < left && TOED_IN_BOUNDS(im.seg_base + q0 + u + 4 <= p.sc.seg_cap, p.sc.words)) dst[u / 4] = d;
     }
 }
 

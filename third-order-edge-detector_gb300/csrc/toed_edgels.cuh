@@ -411,6 +411,7 @@ __device__ __forceinline__ Subpixel subpixel_of(const Staged& e, int W2, bool hy
 static __device__ __noinline__ void band_done(const BatchParams& p, const DetImage& im, int ty, int* s_last)
 {
     __syncthreads();
+    if (!TOED_IN_BOUNDS(im.band_base + ty < p.n_bands, p.sc.words)) return;
     if (threadIdx.x == 0) {
         __threadfence();
         *s_last = atomicAdd(&p.sc.band[im.band_base + ty], 1) == im.nsc - 1;
@@ -420,8 +421,10 @@ static __device__ __noinline__ void band_done(const BatchParams& p, const DetIma
     if (!*s_last) return;
     const long long row = 2LL * p.ed_rows * im.nsc;  // segments a band
     const long long q0 = ty * row, q1 = q0 + row;
+    if (!TOED_IN_BOUNDS(q0 < im.nseg && im.seg_base + im.nseg <= p.sc.seg_cap, p.sc.words)) return;
     const int lo = min(p.sc.seg_dst[im.seg_base + q0], im.cap);
     const int hi = min(q1 < im.nseg ? p.sc.seg_dst[im.seg_base + q1] : *im.count, im.cap);
+    if (!TOED_IN_BOUNDS(lo >= 0, p.sc.words)) return;
     const int per = p.out_f64 ? 2 : 1;  // 16-byte parts of a record
     const uint4* src = static_cast<const uint4*>(im.out);
     uint4* dst = static_cast<uint4*>(im.host_out);
@@ -473,8 +476,10 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
         dst[u] = 0;
         if (r2 < 2 * nrow) {
             const long long q = im.seg_base + (long long)(2 * y0 + r2) * im.nsc + sc;
-            seg[u] = p.sc.seg[q];
-            dst[u] = p.sc.seg_dst[q];
+            if (TOED_IN_BOUNDS(q < im.seg_base + im.nseg && q < p.sc.seg_cap, p.sc.words)) {
+                seg[u] = p.sc.seg[q];
+                dst[u] = p.sc.seg_dst[q];
+            }
         }
         sum += seg[u].y;
     }
@@ -488,6 +493,11 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
     const int px = sc * kInner - E::HALO, py = y0 - E::HALO;
     const int x_al = floor4(px), shift = px - x_al;
     const uint32_t bar = smem_addr(&sBar);
+    // the staged pixels' floats, and whether a window of `side` rows and floats at `win` lies in them
+    [[maybe_unused]] const int n_pix = E::boxes(nrow) * kStepRows * TP;
+    [[maybe_unused]] auto staged = [&](const float* win, int side) {
+        return win >= sPix && (win - sPix) + (side - 1) * TP + side <= n_pix;
+    };
     if (im.tma) {
         if (tid == 0) {
             mbar_init(bar);
@@ -508,7 +518,8 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
                 const Bytes4 b = fetch_bytes(im.src, im.pitch, H, W, py + r, px, lane & 15, E::TW);
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    if (r < nr && (unsigned)(b.c + e) < (unsigned)E::TW)
+                    if (r < nr && (unsigned)(b.c + e) < (unsigned)E::TW &&
+                        TOED_IN_BOUNDS(r * TP + shift + b.c + e < n_pix, p.sc.words))
                         sPix[r * TP + shift + b.c + e] = (float)((b.w >> (8 * e)) & 255u);
             }
         } else {
@@ -518,7 +529,7 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
 #pragma unroll
                 for (int c = 0; c < (E::TW + 31) / 32; ++c) {
                     const int col = lane + 32 * c, y = py + r, x = px + col;
-                    if (col < E::TW)
+                    if (col < E::TW && TOED_IN_BOUNDS(r * TP + shift + col < n_pix, p.sc.words))
                         sPix[r * TP + shift + col] = (unsigned)y < (unsigned)H && (unsigned)x < (unsigned)W
                                                          ? __ldg(src + (long long)y * im.pitch + x)
                                                          : 0.f;
@@ -543,7 +554,7 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
         int pos = -1;
         if (tid < n) {
             const int2 l = sList[tid];
-            if (l.y < cap && l.x < p.sc.staging_cap) {
+            if (l.y < cap && l.x < p.sc.staging_cap && TOED_IN_BOUNDS(l.x >= 0 && l.y >= 0, p.sc.words)) {
                 pos = l.y;
                 e = load_staged(p.sc, l.x);
             }
@@ -567,9 +578,11 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
         if (pos >= 0) {
             const unsigned lt_ = (1u << lane) - 1u;
             const int to = odd ? n0 + (before & 0xffff) + __popc(b1 & lt_) : (before >> 16) + __popc(b0 & lt_);
-            sRec[to] = e;
-            sPos[to] = pos;
-            if (QAD) sAt[to] = at;
+            if (TOED_IN_BOUNDS(to < kEdThreads, p.sc.words)) {
+                sRec[to] = e;
+                sPos[to] = pos;
+                if (QAD) sAt[to] = at;
+            }
         }
         __syncthreads();
         pos = sPos[tid];
@@ -581,6 +594,7 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
             if constexpr (QAD) {
                 const Subpixel q = sAt[pos >= 0 ? tid : (wid * 32)];
                 const float* win = sPix + ((q.Y1 >> 1) - y0 + 1) * TP + (q.X1 >> 1) - sc * kInner + 1 + shift;
+                if (!TOED_IN_BOUNDS(staged(win, NT + 2), p.sc.words)) win = sPix;
                 float d9[9];
                 if (32 * wid < n0)
                     subpixel9<R, 1>(win, q.Y1, (float)q.tx, (float)q.ty, sTab, p.taps, d9);
@@ -592,6 +606,7 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
                 for (int f = 0; f < 7; ++f) d7[f] = d9[f + 2];
             } else {
                 const float* win = sPix + ((Gr >> 1) - y0) * TP + (Gc >> 1) - sc * kInner + shift;
+                if (!TOED_IN_BOUNDS(staged(win, NT), p.sc.words)) win = sPix;
                 if (32 * wid < n0)
                     window7<R, 0>(win, a, sTab + (a ? 2 : b) * NT, p.taps, d7);
                 else
@@ -605,7 +620,8 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
                 ori = (tix == 0.f && tiy == 0.f) ? __int_as_float(0x7fc00000) : atan2f(tix, -tiy);
                 if (pos >= 0 && cancels(gx, gy, d7, tix, tiy)) {
                     sPos[tid] = -2 - pos;
-                    sFlag[atomicAdd(&sFlags, 1)] = (unsigned char)tid;
+                    const int f = atomicAdd(&sFlags, 1);
+                    if (TOED_IN_BOUNDS(f < kEdThreads, p.sc.words)) sFlag[f] = (unsigned char)tid;
                 }
             } else {
                 const float fxx = d7[0], fxy = d7[1], fyy = d7[2], fxxy = d7[3], fxyy = d7[4], fxxx = d7[5], fyyy = d7[6];
@@ -626,23 +642,27 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
             for (int f = f0; f < nf && m < kRefineMost; f += kEdThreads / 32, ++m) {
                 if constexpr (QAD) {
                     const Subpixel q = sAt[sFlag[f]];
-                    refine_subpixel(p, sPix + ((q.Y1 >> 1) - y0 + 1) * TP + (q.X1 >> 1) - sc * kInner + 1 + shift, TP,
-                                    q.X1, q.Y1, q.tx, q.ty, lane, sD64[wid][m]);
+                    const float* win = sPix + ((q.Y1 >> 1) - y0 + 1) * TP + (q.X1 >> 1) - sc * kInner + 1 + shift;
+                    if (TOED_IN_BOUNDS(staged(win, NT + 2), p.sc.words))
+                        refine_subpixel(p, win, TP, q.X1, q.Y1, q.tx, q.ty, lane, sD64[wid][m]);
                 } else {
                     const int idx = sRec[sFlag[f]].idx;
                     const int Gr = idx / W2, Gc = idx - Gr * W2;
-                    refine_edgel(p, sPix + ((Gr >> 1) - y0) * TP + (Gc >> 1) - sc * kInner + shift, TP, Gr & 1, Gc & 1,
-                                 lane, sD64[wid][m]);
+                    const float* win = sPix + ((Gr >> 1) - y0) * TP + (Gc >> 1) - sc * kInner + shift;
+                    if (TOED_IN_BOUNDS(staged(win, NT), p.sc.words))
+                        refine_edgel(p, win, TP, Gr & 1, Gc & 1, lane, sD64[wid][m]);
                 }
             }
             __syncwarp();
             if (lane < m) {
                 const int pos = -2 - sPos[sFlag[f0 + lane * (kEdThreads / 32)]];
                 const float ori = orientation64(sD64[wid][lane]);
-                if (p.out_f64)
-                    static_cast<double*>(im.out)[4LL * pos + 2] = (double)ori;
-                else
-                    static_cast<float*>(im.out)[4LL * pos + 2] = ori;
+                if (TOED_IN_BOUNDS(pos >= 0 && pos < cap, p.sc.words)) {
+                    if (p.out_f64)
+                        static_cast<double*>(im.out)[4LL * pos + 2] = (double)ori;
+                    else
+                        static_cast<float*>(im.out)[4LL * pos + 2] = ori;
+                }
             }
             __syncwarp();
         }
