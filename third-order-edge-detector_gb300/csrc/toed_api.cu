@@ -604,12 +604,12 @@ static toed_status check_batch(const toed_ctx* c, const toed_image* images, int 
 // The batch in chunks of kBatchMax images (caller holds c->mu, device set).
 static toed_status detect_all(toed_ctx* c, const toed_image* images, int n, const toed_params* prm,
                               cudaStream_t stream, const toed_tuning* force = nullptr, const int* wait_slot = nullptr,
-                              const HostList* hosts = nullptr, bool first = true)
+                              const HostList* hosts = nullptr)
 {
     const int r = radius_of(prm);
     toed_status st = TOED_OK;
     for (int i0 = 0; i0 < n && st == TOED_OK; i0 += kBatchMax)
-        st = detect_chunk(c, images + i0, std::min(kBatchMax, n - i0), prm, r, first && i0 == 0, stream, force,
+        st = detect_chunk(c, images + i0, std::min(kBatchMax, n - i0), prm, r, i0 == 0, stream, force,
                           wait_slot ? wait_slot + i0 : nullptr, hosts ? hosts + i0 : nullptr);
     return st;
 }
@@ -718,13 +718,6 @@ extern "C" toed_status toed_detect(toed_ctx* c, const toed_image* image, const t
 {
     return toed_detect_batch(c, image, 1, prm, stream);
 }
-
-// Host batches are cut in two pipelines after this share of the pixels, if at
-// least so many are left.  64 images, 79 Mpixel: 2.42 ms in one, 2.30 cut at
-// 50 or 60 %, 2.44 at 80; below these sizes the second pipeline's launches cost
-// what it hides.
-constexpr int kHostCutPercent = 55;
-constexpr long long kHostCutPixels = 4 << 20;
 
 // Launches run one at a time, each waited for: CUDA_LAUNCH_BLOCKING=1, or a
 // tool injected into the runtime (profilers and checkers serialise work).
@@ -944,33 +937,7 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
         const int early = std::min(chunks, 2);
         for (int k = 0; k < early; ++k) TOED_HB(enqueue_group(k));
         TOED_HB(preload_finalize(radius_of(prm), prm->orientation == TOED_ORI_QAD));
-        // two launches of the whole pipeline where there is something to
-        // overlap: the first images' edgels are finished, and cross to the host,
-        // while the last images' pixels are still arriving.  The scratch is
-        // grown for both before the first, since growing waits for the device.
-        int cut = n;
-        {
-            long long px = 0;
-            for (int i = 0; i + 1 < n && cut == n; ++i) {
-                px += (long long)images[i].height * images[i].width;
-                if (px * 100 >= total_px * kHostCutPercent && total_px - px >= kHostCutPixels) cut = i + 1;
-            }
-        }
-        if (cut < n) {
-            long long segs = 0, bands = 0, cap = 0;
-            for (int i = 0; i < n; ++i) {
-                const long long nseg = 2LL * images[i].height * ((images[i].width + kInner - 1) / kInner);
-                segs += (nseg + kScanTileMax - 1) / kScanTileMax * kScanTileMax;
-                bands += images[i].height;
-                cap += images[i].capacity;
-            }
-            st = ensure_scratch(c, staging_records(cap, most_warps(c)), segs, segs / kSegTile, n, stream);
-            if (st == TOED_OK && direct) st = grow(&c->band, &c->band_cap, bands, stream);
-        }
-        const HostList* hl = direct ? lists.data() : nullptr;
-        if (st == TOED_OK) st = detect_all(c, dev.data(), cut, prm, stream, nullptr, slot.data(), hl);
-        if (st == TOED_OK && cut < n)
-            st = detect_all(c, dev.data() + cut, n - cut, prm, stream, nullptr, slot.data() + cut, hl ? hl + cut : nullptr, false);
+        st = detect_all(c, dev.data(), n, prm, stream, nullptr, slot.data(), direct ? lists.data() : nullptr);
         c->ready_spins = kReadySpinLimit;
         if (st != TOED_OK) return fail(st);
         TOED_HB(cudaMemcpyAsync(c->hb_cnt + n, c->words + 2, sizeof(int), cudaMemcpyDeviceToDevice, stream));
