@@ -236,13 +236,17 @@ toed_status toed_detect_noalloc(const toed_image* image, const toed_params* para
  * the launch -- another host thread that waits for the whole device in that
  * moment (cudaDeviceSynchronize, cudaFree) can hold those copies back until
  * the wait gives up (TOED_ERR_TIMEOUT), so serialise such calls; with
- * CUDA_LAUNCH_BLOCKING or under a profiler this flow is not used.  Pageable
+ * CUDA_LAUNCH_BLOCKING or under a profiler this flow is not used.  With
+ * chunks <= 1 page-locked images cross one by one (four groups above 64
+ * images).  Page-locked images that device memory has no room for are read in
+ * place through their device mapping, more slowly.  Pageable
  * images, or more than 64: one launch per group (streams of the context,
  * ordered by events).  Page-locked output buffers (edgels, count, grid_index)
- * are written by a kernel through their device mapping once the lists are
- * complete; pageable ones are filled by copies per group once its
- * counts are read back.  Synchronous: returns when every count and list is in
- * host memory.  Device staging is kept in the context and grows on demand.
+ * are written by a kernel through their device mapping, each list band by band
+ * as its bands are finished: they are partly written during the call, and valid
+ * only when it returns TOED_OK; pageable ones are filled by copies per group
+ * once its counts are read back.  Synchronous: returns when every count and list
+ * is in host memory.  Device staging is kept in the context and grows on demand.
  * Page-locked image buffers give full copy speed.  Returns
  * TOED_ERR_TIMEOUT if a bounded device wait gave up; more edgels than
  * `capacity` show as count > capacity (the list holds the first capacity). */

@@ -47,10 +47,8 @@ def test_one_launch_for_a_large_batch(toed, synth, pin, f64):
             assert torch.equal(o["index"][:n], r["index"].cpu())
 
 
-def test_lost_copy_in_a_large_batch(toed):
-    """Group 7's ready flag is withheld on the host: the call returns the
-    time-out within its bound, the other images keep their edgels, and the next
-    call succeeds."""
+def _child(body, **env):
+    """Runs `body` in a process of its own (the library reads the injections' variables there)."""
     code = f"""
 import os, sys, time
 sys.path.insert(0, {os.path.dirname(os.path.abspath(__file__))!r})
@@ -61,8 +59,18 @@ from test_gpu_host_launch import SIZES, _batch
 import importlib
 synth = importlib.import_module("toed_gb300.synth")
 det = toed.Detector(0)
-host = _batch(synth, SIZES)
 prm = toed.make_params(1.5)
+host = _batch(synth, SIZES)
+""" + body
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, env=dict(os.environ, **env))
+    assert r.returncode == 0 and "OK" in r.stdout, r.stderr[-3000:]
+
+
+def test_lost_copy_in_a_large_batch(toed):
+    """Group 7's ready flag is withheld on the host: the call returns the
+    time-out within its bound, the other images keep their edgels, and the next
+    call succeeds."""
+    _child("""
 ref = [r["count"] for r in det.detect_batch([im.cuda() for im in host], sigma=1.5)]
 outs = det.alloc_host_outputs(SIZES, capacity=400000)
 os.environ["TOED_TEST_WITHHOLD_READY"] = "7"
@@ -80,6 +88,47 @@ del os.environ["TOED_TEST_WITHHOLD_READY"], os.environ["TOED_TEST_READY_SPINS"]
 det.detect_host(host, outs, prm)
 assert [int(o["count"].item()) for o in outs] == ref
 print("OK")
-"""
-    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
-    assert r.returncode == 0 and "OK" in r.stdout, r.stderr[-3000:]
+""")
+
+
+def test_one_group_asked_for_crosses_in_several(toed):
+    """chunks = 1: more groups are used, so that detection starts before the
+    last pixel is in -- seen by withholding the second group's flag."""
+    _child("""
+outs = det.alloc_host_outputs(SIZES, capacity=400000)
+try:
+    det.detect_host(host, outs, prm, chunks=1)
+    raise SystemExit("one group")
+except toed.ToedError as e:
+    assert e.status == toed.TOED_ERR_TIMEOUT, e
+print("OK")
+""", TOED_TEST_WITHHOLD_READY="1", TOED_TEST_READY_SPINS="4096")
+
+
+@pytest.mark.parametrize("chunks", [1, 5])
+def test_no_device_memory_for_the_pixels(toed, chunks):
+    """Page-locked images are read in place when device memory for them cannot
+    be had: float32 and 8-bit, rows off 16-byte boundaries, lists as ever."""
+    _child(f"""
+wide = torch.zeros((1400, 1503), dtype=torch.float32).pin_memory()
+wide[:, 1:1501] = host[1][:900].repeat(2, 1)[:1400, :1500]
+ims = host + [wide[:, 1:1501], host[4].round().to(torch.uint8).pin_memory(), host[5].round().to(torch.uint8).pin_memory()]
+ref = det.detect_batch([im.contiguous().cuda() for im in ims], sigma=1.5)
+ref = [(r["count"], r["edgels"].cpu(), r["index"].cpu()) for r in ref]
+outs = det.alloc_host_outputs([tuple(im.shape) for im in ims], capacity=400000, index=True)
+for k in range(2):
+    det.detect_host(ims, outs, prm, chunks={chunks})
+    for (n, e, i), o in zip(ref, outs):
+        assert int(o["count"].item()) == n and torch.equal(o["edgels"][:n], e) and torch.equal(o["index"][:n], i)
+det.close()
+torch.cuda.empty_cache()
+# a fresh context, a threshold that nothing reaches: no staging for the 107 MB of pixels is held
+det = toed.Detector(0)
+outs = det.alloc_host_outputs([tuple(im.shape) for im in ims], capacity=2000)
+torch.cuda.synchronize()
+free = torch.cuda.mem_get_info()[0]
+det.detect_host(ims, outs, toed.make_params(1.5, threshold=1e6), chunks={chunks})
+held = free - torch.cuda.mem_get_info()[0]
+assert held < 60e6, held
+print("OK")
+""", TOED_TEST_NO_STAGING="1")

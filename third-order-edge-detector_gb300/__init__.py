@@ -257,7 +257,7 @@ class HostBatch:
         self.arr = arr
 
     def run(self, params: toed_params, chunks=None, stream=None):
-        """chunks: copy groups (None: one image per group, the fastest for
+        """chunks: copy groups (None or 1: one image per group, the fastest for
         page-locked images)."""
         det = self.det
         if chunks is None:

@@ -428,11 +428,13 @@ struct HostList {
 };
 
 // hosts (optional, per image): where the finished list goes.
+// in_place: the pixels are page-locked host memory, read through its mapping (by loads)
 // wait_slot (optional, per image): 0, or g > 0 when the copy engine is still
 // bringing the image in and c->hb_ready[g - 1] == c->hb_epoch marks its arrival
 static toed_status detect_chunk(toed_ctx* c, const toed_image* images, int n, const toed_params* prm,
                                 int r, bool first_chunk, cudaStream_t stream, const toed_tuning* force = nullptr,
-                                const int* wait_slot = nullptr, const HostList* hosts = nullptr)
+                                const int* wait_slot = nullptr, const HostList* hosts = nullptr,
+                                bool in_place = false)
 {
     const bool hyb = prm->precision != TOED_FP32;
     const bool nmsto = prm->nms_direction == TOED_NMS_TO_NORMAL;
@@ -518,7 +520,7 @@ static toed_status detect_chunk(toed_ctx* c, const toed_image* images, int n, co
         d.seg_base = tiles * seg_tile;
         d.ed_base = (int)ed;
         d.wait_slot = wait_slot ? wait_slot[i] : 0;
-        if (use && use->staging != 1)
+        if ((use && use->staging != 1) || in_place)
             d.tma = 0;  // loads prefetched in registers
         else
             encode_rows_map(&p->tmap[i], d, r);  // TMA where the image allows it (a host call per image)
@@ -604,13 +606,13 @@ static toed_status check_batch(const toed_ctx* c, const toed_image* images, int 
 // The batch in chunks of kBatchMax images (caller holds c->mu, device set).
 static toed_status detect_all(toed_ctx* c, const toed_image* images, int n, const toed_params* prm,
                               cudaStream_t stream, const toed_tuning* force = nullptr, const int* wait_slot = nullptr,
-                              const HostList* hosts = nullptr)
+                              const HostList* hosts = nullptr, bool in_place = false)
 {
     const int r = radius_of(prm);
     toed_status st = TOED_OK;
     for (int i0 = 0; i0 < n && st == TOED_OK; i0 += kBatchMax)
         st = detect_chunk(c, images + i0, std::min(kBatchMax, n - i0), prm, r, i0 == 0, stream, force,
-                          wait_slot ? wait_slot + i0 : nullptr, hosts ? hosts + i0 : nullptr);
+                          wait_slot ? wait_slot + i0 : nullptr, hosts ? hosts + i0 : nullptr, in_place);
     return st;
 }
 
@@ -769,7 +771,6 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
         dev[i].dtype = h.dtype;
         dev[i].capacity = h.capacity;
     }
-    chunks = std::max(1, std::min(chunks, n));
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     TOED_CU(cudaStreamIsCapturing(stream, &cs));
     if (cs != cudaStreamCaptureStatusNone) return TOED_ERR_CAPTURE;
@@ -778,8 +779,6 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
     if (prev != c->device) TOED_CU(cudaSetDevice(c->device));
     std::lock_guard<std::mutex> lk(c->mu);
     toed_status st = TOED_OK;
-    std::vector<cudaEvent_t> ev_in(chunks, nullptr), ev_det(chunks, nullptr);
-    std::vector<int> first(chunks + 1, n);
     auto fail = [&](toed_status s) {
         // an early return must not leave copies in flight: the next call
         // reuses the staging and rewrites the epoch their flag copies read
@@ -814,14 +813,34 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
     // drains the GPU.  Pageable inputs: staged copies per group, one
     // detection launch per group once its copy is in.
     bool zin = true;
-    for (int i = 0; i < n && zin; ++i) zin = mapped(const_cast<void*>(images[i].pixels)) != nullptr;
+    std::vector<const void*> in_map(n, nullptr);
+    for (int i = 0; i < n && zin; ++i) {
+        in_map[i] = mapped(const_cast<void*>(images[i].pixels));
+        zin = in_map[i] != nullptr;
+    }
+    // Asked for one group, page-locked images still cross in several: one group
+    // leaves nothing to overlap (64 images, 79 Mpixel: 3.70 ms a call, 2.49 with
+    // an image a group), and the lists are the same.  Beyond one launch's images
+    // a group costs launches of its own.
+    if (zin && chunks <= 1) chunks = n <= kBatchMax ? n : 4;
+    chunks = std::max(1, std::min(chunks, n));
+    // Page-locked images that device memory has no room for are read in place
+    // through their mapping (by loads, and twice over the link: 6.5 ms).
+    // TOED_TEST_NO_STAGING: as if it had none (failure injection for tests).
+    bool inplace = zin && std::getenv("TOED_TEST_NO_STAGING");
+    if (!inplace && (st = grow(&c->hb_in, &c->hb_in_cap, std::max(in_b, 1LL), stream)) != TOED_OK) {
+        inplace = zin && cudaGetLastError() == cudaErrorMemoryAllocation;
+        if (!inplace) return fail(st);
+    }
+    if (inplace) chunks = 1;
+    std::vector<cudaEvent_t> ev_in(chunks, nullptr), ev_det(chunks, nullptr);
+    std::vector<int> first(chunks + 1, n);
     // (flagged: one launch of at most kBatchMax images, so that nothing between
     // the launch and the copies' enqueueing can wait for the device; never
     // when launches run serialised -- CUDA_LAUNCH_BLOCKING, or a profiler or
     // checker injected into the runtime -- since then the waiting launch
     // would hold the host or the device until its wait gives up)
-    const bool flagged = zin && n <= kBatchMax && !launches_serialised();
-    if ((st = grow(&c->hb_in, &c->hb_in_cap, std::max(in_b, 1LL), stream)) != TOED_OK) return fail(st);
+    const bool flagged = zin && !inplace && n <= kBatchMax && !launches_serialised();
     if (flagged) {
         const long long had = c->hb_ready_cap;
         if ((st = grow(&c->hb_ready, &c->hb_ready_cap, (long long)chunks, stream)) != TOED_OK) return fail(st);
@@ -846,7 +865,8 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
     bool direct = true;
     std::vector<HostList> lists(n);
     for (int i = 0; i < n; ++i) {
-        dev[i].pixels = c->hb_in + in_off[i];
+        dev[i].pixels = inplace ? in_map[i] : c->hb_in + in_off[i];
+        if (inplace) dev[i].pitch = images[i].pitch;
         dev[i].edgels = c->hb_out + out_off[i];
         dev[i].count = c->hb_cnt + i;
         dev[i].grid_index = images[i].grid_index ? c->hb_idx + idx_off[i] : nullptr;
@@ -947,15 +967,15 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
         first[1] = n;
     } else {
         // 1. every group's images to the device, in order
-        for (int k = 0; k < chunks; ++k) {
+        for (int k = 0; k < chunks && !inplace; ++k) {
             TOED_HB(copy_group(k));
             TOED_HB(cudaEventRecord(ev_in[k], c->s_in));
         }
         // 2. detection of each group once its images are in
         for (int k = 0; k < chunks; ++k) {
-            TOED_HB(cudaStreamWaitEvent(stream, ev_in[k], 0));
+            if (!inplace) TOED_HB(cudaStreamWaitEvent(stream, ev_in[k], 0));
             st = detect_all(c, dev.data() + first[k], first[k + 1] - first[k], prm, stream, nullptr, nullptr,
-                            direct ? lists.data() + first[k] : nullptr);
+                            direct ? lists.data() + first[k] : nullptr, inplace);
             if (st != TOED_OK) return fail(st);
             TOED_HB(cudaMemcpyAsync(c->hb_cnt + n + k, c->words + 2, sizeof(int), cudaMemcpyDeviceToDevice, stream));
             TOED_HB(cudaEventRecord(ev_det[k], stream));
