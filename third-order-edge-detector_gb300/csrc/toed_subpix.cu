@@ -457,19 +457,11 @@ __global__ void __launch_bounds__(256, 5) tc_orient_nms(const __grid_constant__ 
             } else {
                 s2 = second_border(sSmI, i, j, h, w, i0, j0);
             }
-            float x, y;
-            if (sE[a + HE][b + HE] > p.thresh) {
-                const float sgn = (s2.xy < 0) ? 1.f : ((s2.xy > 0) ? -1.f : 0.f);
-                constexpr double kEps = 1e-5;
-                constexpr float kEpsHi = (float)kEps, kEpsLo = (float)(kEps - (double)kEpsHi);
-                x = df_add(df_second(s2.xx, down), make_float2(kEpsHi, kEpsLo)).x;
-                y = df_second(s2.yy, down).x * sgn;
-            } else {  // no candidate: its direction is a weight, a rounding or two of the scaling do not matter
-                const float k = down * (1.f / 2500.f);
-                x = fmaf(__ll2float_rn(s2.xx), k, 1e-5f);
-                y = __ll2float_rn(s2.xy < 0 ? s2.yy : -s2.yy) * k;
-                if (s2.xy == 0) y = 0.f;
-            }
+            const float sgn = (s2.xy < 0) ? 1.f : ((s2.xy > 0) ? -1.f : 0.f);
+            constexpr double kEps = 1e-5;
+            constexpr float kEpsHi = (float)kEps, kEpsLo = (float)(kEps - (double)kEpsHi);
+            const float x = df_add(df_second(s2.xx, down), make_float2(kEpsHi, kEpsLo)).x;
+            const float y = df_second(s2.yy, down).x * sgn;
             const float2 d = x != 0.f ? hessian_dir(x, y) : hessian_dir0(x, y);
             sDir[a][b] = d;
             p.dir[M.px_base + (long long)i * w + j] = d;
