@@ -209,7 +209,7 @@ toed_status toed_subpix_to_correct_batch(toed_ctx* ctx, const toed_edgemap* maps
  * grows on demand.  One image per call on the current device; the caller
  * passes the image and the output buffers as for toed_detect, and the same
  * image checks apply.  The scratch is a fixed array compiled into the
- * library (about 11 MB).  The CUDA runtime loads it lazily: the first call
+ * library (about 12 MB).  The CUDA runtime loads it lazily: the first call
  * on a device reserves it there (until the process exits) and looks up its
  * device address, so make that first call at start-up, before a pool or
  * arena claims the device's memory (else TOED_ERR_CUDA) and before any

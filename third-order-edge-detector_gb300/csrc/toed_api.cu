@@ -141,20 +141,22 @@ struct toed_ctx {
     int num_sms = 0;
     int* words = nullptr;  // kWords: [0] queue [1] cursor [2] flags [3] tile ticket [4] debug
     double4_32a* staging = nullptr;
-    int* staging_idx = nullptr;
     long long staging_cap = 0;
     int2* seg = nullptr;
     long long seg_cap = 0;
-    int* tile_sum = nullptr;
-    long long tile_cap = 0;
-    long long* img_base = nullptr;
-    int img_cap = 0;
     int* seg_dst = nullptr;
     long long dst_cap = 0;
     int* band = nullptr;
     long long band_cap = 0;
     unsigned long long* tile_state = nullptr;  // the scan's tiles
     long long state_cap = 0;
+    // TO correction
+    int* staging_idx = nullptr;
+    long long idx_cap = 0;
+    int* tile_sum = nullptr;
+    long long tile_cap = 0;
+    long long* img_base = nullptr;
+    long long img_cap = 0;
     float2* dir = nullptr;
     int* eid = nullptr;
     int* win = nullptr;
@@ -311,23 +313,18 @@ static toed_status grow(T** buf, long long* cap, long long need, cudaStream_t st
     return TOED_OK;
 }
 
-static toed_status ensure_scratch(toed_ctx* c, long long staging, long long segs, long long tiles,
-                                  int imgs, cudaStream_t stream)
+// What the detection and the TO correction both use, then what the detection
+// alone does.
+static toed_status ensure_staging(toed_ctx* c, long long staging, long long segs, cudaStream_t stream)
 {
-    toed_status st;
-    long long sc = c->staging_cap;
-    if ((st = grow(&c->staging, &sc, staging, stream)) != TOED_OK) return st;
-    long long sc2 = c->staging_cap;
-    if ((st = grow(&c->staging_idx, &sc2, staging, stream)) != TOED_OK) return st;
-    c->staging_cap = std::min(sc, sc2);
-    if ((st = grow(&c->seg, &c->seg_cap, segs, stream)) != TOED_OK) return st;
-    if ((st = grow(&c->seg_dst, &c->dst_cap, segs, stream)) != TOED_OK) return st;
-    if ((st = grow(&c->tile_sum, &c->tile_cap, tiles, stream)) != TOED_OK) return st;
-    if ((st = grow(&c->tile_state, &c->state_cap, tiles, stream)) != TOED_OK) return st;
-    long long ic = c->img_cap;
-    if ((st = grow(&c->img_base, &ic, (long long)imgs, stream)) != TOED_OK) return st;
-    c->img_cap = (int)ic;
-    return TOED_OK;
+    const toed_status st = grow(&c->staging, &c->staging_cap, staging, stream);
+    return st == TOED_OK ? grow(&c->seg, &c->seg_cap, segs, stream) : st;
+}
+static toed_status ensure_scratch(toed_ctx* c, long long staging, long long segs, long long tiles, cudaStream_t stream)
+{
+    toed_status st = ensure_staging(c, staging, segs, stream);
+    if (st == TOED_OK) st = grow(&c->seg_dst, &c->dst_cap, segs, stream);
+    return st == TOED_OK ? grow(&c->tile_state, &c->state_cap, tiles, stream) : st;
 }
 
 // Staging records that `edgels` survivors of `warps` warps can take.  A warp
@@ -354,7 +351,7 @@ extern "C" toed_status toed_reserve(toed_ctx* c, long long max_pixels, long long
     const long long segs = max_pixels / 15 + 2LL * 4096 + (long long)imgs * kScanTileMax;
     const long long tiles = segs / kSegTile + imgs + 1;
     std::lock_guard<std::mutex> lk(c->mu);
-    toed_status st = ensure_scratch(c, staging_records(max_edgels, most_warps(c)), segs, tiles, imgs, nullptr);
+    toed_status st = ensure_scratch(c, staging_records(max_edgels, most_warps(c)), segs, tiles, nullptr);
     cudaSetDevice(prev);
     return st;
 }
@@ -544,16 +541,13 @@ static toed_status detect_chunk(toed_ctx* c, const toed_image* images, int n, co
     p->n_tiles = (int)tiles;
     p->stage_blk = kStageBlk;
     const long long records = staging_records(staging, resident * (kThreads / 32));
-    toed_status st = ensure_scratch(c, records, tiles * seg_tile, tiles, n, stream);
+    toed_status st = ensure_scratch(c, records, tiles * seg_tile, tiles, stream);
     if (st != TOED_OK) return st;
     p->sc.words = c->words;
     p->sc.staging = c->staging;
-    p->sc.staging_idx = c->staging_idx;
     p->sc.staging_cap = c->staging_cap;
     p->sc.seg = c->seg;
     p->sc.seg_cap = c->seg_cap;
-    p->sc.tile_sum = c->tile_sum;
-    p->sc.img_base = c->img_base;
     if (p->n_bands > 0 && (st = grow(&c->band, &c->band_cap, (long long)p->n_bands, stream)) != TOED_OK) return st;
     p->sc.band = c->band;
     p->sc.seg_dst = c->seg_dst;
@@ -1114,18 +1108,22 @@ extern "C" toed_status toed_subpix_to_correct_batch(toed_ctx* c, const toed_edge
                 if (sc > 1) work += hw * (mp[i].theta ? 2 : 1);
             }
             segs = segtiles * kSegTile;
-            if ((st = ensure_scratch(c, stag, segs, segtiles, cn, stream)) != TOED_OK) break;
+            if ((st = ensure_staging(c, stag, segs, stream)) != TOED_OK) break;
+            if ((st = grow(&c->staging_idx, &c->idx_cap, stag, stream)) != TOED_OK) break;
+            if ((st = grow(&c->tile_sum, &c->tile_cap, segtiles, stream)) != TOED_OK) break;
+            if ((st = grow(&c->img_base, &c->img_cap, (long long)cn, stream)) != TOED_OK) break;
             if ((st = grow(&c->dir, &c->px_cap, px, stream)) != TOED_OK) break;
             if ((st = grow(&c->eid, &c->px_cap2, px, stream)) != TOED_OK) break;
-            if ((st = grow(&c->win, &c->px_cap3, px, stream)) != TOED_OK) break;
+            // (the winners of the dense maps on a work grid)
+            if (sc > 1 && (st = grow(&c->win, &c->px_cap3, px, stream)) != TOED_OK) break;
             if ((st = grow(&c->img_count, &c->img_count_cap, (long long)cn, stream)) != TOED_OK) break;
-            if ((st = grow(&c->keep, &c->keep_cap, c->staging_cap, stream)) != TOED_OK) break;
+            if ((st = grow(&c->keep, &c->keep_cap, stag, stream)) != TOED_OK) break;
             if (work > 0 && (st = grow(&c->sp_work, &c->sp_work_cap, work, stream)) != TOED_OK) break;
             SubScratch s;
             s.sc.words = c->words;
             s.sc.staging = c->staging;
             s.sc.staging_idx = c->staging_idx;
-            s.sc.staging_cap = std::min(c->staging_cap, c->keep_cap);
+            s.sc.staging_cap = std::min({c->staging_cap, c->idx_cap, c->keep_cap});
             s.sc.seg = c->seg;
             s.sc.seg_cap = c->seg_cap;
             s.sc.tile_sum = c->tile_sum;

@@ -4,10 +4,10 @@
 // Data layout in HBM (all caller-owned except the scratch block):
 //   image k      : H x pitch pixels (uint8 or float32), row-major
 //   edgels k     : capacity x 4 (float32 or float64) [x, y, orientation, strength]
-//   scratch      : work-queue / cursor / flags words, staging records
-//                  (double4 + int index per edgel), the row-segment table
-//                  (int2 {staging offset, count} per (2x-grid row, strip column)),
-//                  and the ordering pass' tile sums.
+//   scratch      : work-queue / cursor / flags words, staging records (32 bytes
+//                  an edgel), the row-segment table (int2 {staging offset, count}
+//                  per (2x-grid row, strip column)), each segment's place in its
+//                  list, and a word per tile of the scan.
 #pragma once
 #include <cstdint>
 #include <cuda.h>  // CUtensorMap (the type only; encoding goes through the runtime's driver entry point)
@@ -108,12 +108,12 @@ struct Scratch {
                          // ticket, [4] (bounds-checked builds) source line of the first failed check
     double4_32a* staging;  // staged edgels, 32 bytes each: TO correction (x, y, orientation, strength);
                            // the detection two float4 (det_stage)
-    int* staging_idx;
+    int* staging_idx;      // TO correction: pixel of each staged edgel
     long long staging_cap;
     int2* seg;           // per segment {staging offset, count}
     long long seg_cap;   // segments `seg` holds
-    int* tile_sum;       // per ordering tile
-    long long* img_base; // per image: exclusive prefix of its first segment
+    int* tile_sum;       // TO correction: per ordering tile
+    long long* img_base; // TO correction: per map, exclusive prefix of its first segment
     int* band;           // per band of an image with host_out: edgel-kernel tiles done
     int* seg_dst;        // per segment: its place in its image's list
     unsigned long long* tile_state;  // per scan tile: {0, 1 its count, 2 the count of its image's

@@ -8,8 +8,8 @@
 // pre-sized buffers) -- and so cannot create a toed_ctx, whose scratch grows
 // with cudaMalloc on demand.
 //
-// How: the scratch the fused kernel and the ordering pass need (work-queue
-// and flag words, staged edgel records, the row-segment table, tile sums)
+// How: the scratch that a detection's kernels need (work-queue and flag
+// words, staged edgel records, the row-segment table, the scan's words)
 // lives in one file-scope __device__ array of fixed size, g_noalloc_scratch.
 // The CUDA runtime loads the module that holds it lazily (the default since
 // CUDA 12): the bytes are reserved on a device when the first call on that
@@ -52,15 +52,12 @@ constexpr long long kNaMaxSegs = kNaMaxTiles * kSegTile;
 constexpr size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 constexpr size_t kOffWords = 0;
 constexpr size_t kOffStaging = align256(kOffWords + kWords * sizeof(int));
-constexpr size_t kOffIdx = align256(kOffStaging + sizeof(double4_32a) * kNaMaxEdgels);
-constexpr size_t kOffSeg = align256(kOffIdx + sizeof(int) * kNaMaxEdgels);
+constexpr size_t kOffSeg = align256(kOffStaging + sizeof(double4_32a) * kNaMaxEdgels);
 constexpr size_t kOffDst = align256(kOffSeg + sizeof(int2) * kNaMaxSegs);
-constexpr size_t kOffTiles = align256(kOffDst + sizeof(int) * kNaMaxSegs);
-constexpr size_t kOffBase = align256(kOffTiles + sizeof(int) * kNaMaxTiles);
-constexpr size_t kOffState = align256(kOffBase + sizeof(long long));
+constexpr size_t kOffState = align256(kOffDst + sizeof(int) * kNaMaxSegs);
 constexpr size_t kScratchBytes = align256(kOffState + sizeof(unsigned long long) * kNaMaxTiles);
 
-// The fixed scratch (see the file comment): about 11 MB per device.
+// The fixed scratch (see the file comment): about 12 MB per device.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
 constexpr int kMaxDevices = 64;
@@ -192,12 +189,9 @@ extern "C" toed_status toed_detect_noalloc(const toed_image* im, const toed_para
     p.n_tiles = (int)((d.nseg + kSegTile - 1) / kSegTile);
     p.sc.words = reinterpret_cast<int*>(base + kOffWords);
     p.sc.staging = reinterpret_cast<double4_32a*>(base + kOffStaging);
-    p.sc.staging_idx = reinterpret_cast<int*>(base + kOffIdx);
     p.sc.staging_cap = im->capacity > 0 ? im->capacity : 1;
     p.sc.seg = reinterpret_cast<int2*>(base + kOffSeg);
     p.sc.seg_cap = kNaMaxSegs;
-    p.sc.tile_sum = reinterpret_cast<int*>(base + kOffTiles);
-    p.sc.img_base = reinterpret_cast<long long*>(base + kOffBase);
     p.sc.seg_dst = reinterpret_cast<int*>(base + kOffDst);
     p.sc.tile_state = reinterpret_cast<unsigned long long*>(base + kOffState);
 
