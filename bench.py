@@ -12,10 +12,11 @@ detection pass over the whole batch (detection, scan and edgel kernels).
 * ``e2e``     : the same metric through the public API with host buffers:
                 each step copies the images from pinned host memory, detects,
                 and reads back the counts and the edgel lists.
-* ``roofline``: the fused kernel is FP32-FMA-issue bound (a separable
-                stencil, no tensor cores); achieved FP32 rate of its dense
-                work against the FP32 FMA rate measured in the same run, plus
-                the HBM fraction of its algorithmic bytes.
+* ``roofline``: the whole step's algorithmic bytes (images in, lists and counts
+                out) over the step's time, against the measured HBM copy rate;
+                beside it the roof that binds, FP32 FMA issue: the dense kernel's
+                executed work over that kernel's own time, against the FMA rate
+                measured in the same run.
 * ``cpu_baseline``: the oracle restatement of the reference's OpenMP FP64
                 CPU path on the host cores, on a bounded sample.
 
@@ -630,6 +631,22 @@ def flops_per_px(r: int) -> int:
     return 64 * r + 88
 
 
+def hbm_roofline(npx, n_edgels, n_images, step_ms, peak):
+    """The step against HBM: float32 pixels read once, 16 bytes an edgel and a
+    count an image written once, over the time of all three kernels; and the
+    DRAM bytes these moved in the committed ncu capture, scaled by pixels."""
+    alg = npx * 4 + n_edgels * 16 + 4 * n_images
+    ach = alg / (step_ms * 1e-3) / 1e9
+    traffic = None
+    tf = os.path.join(ROOT, "profiles", "toed_detect_kernel__uneven_batch64_sigma1.5.traffic.txt")
+    if os.path.exists(tf):
+        kv = dict(line.split() for line in open(tf) if line.strip() and not line.startswith("#"))
+        traffic = int(int(kv["dram_bytes_per_step"]) * npx / int(kv["pixels"]))
+    return {"bound": "hbm", "achieved": round(ach, 2), "peak": peak, "unit": "GB/s", "frac": round(ach / peak, 5),
+            "traffic": traffic, "bytes_per_px": round(alg / npx, 4),
+            "traffic_bytes_per_px": round(traffic / npx, 3) if traffic else None}
+
+
 def run_ours(args, ws, rank, local):
     seed0 = SEED0 + N_IMAGES * rank
     images = make_batch(seed0)  # spawn pool, before the first CUDA call
@@ -668,15 +685,15 @@ def run_ours(args, ws, rank, local):
     if det.flags(stream) != 0:
         raise RuntimeError("capacity exceeded in the warm-up")
     # the detection kernel's own duration (library-side CUDA events on the
-    # launching stream), for the roofline
+    # launching stream), for its FP32 rate
     det.profile_begin()
     for s in range(args.steps):
         det.detect_into(d_imgs, outs, params, stream)
     torch.cuda.synchronize()
     ksum, klaunch = det.profile_end()
     kernel_ms = ksum / max(klaunch, 1)
-    # the step as deployed: the whole batch (persistent detection launch and
-    # the ordering pass) captured once in a CUDA graph and replayed
+    # the step as deployed: the whole batch (detection, scan and edgel kernels)
+    # captured once in a CUDA graph and replayed
     graph = det.capture(d_imgs, outs, params)
     for _ in range(args.warmup):
         graph.replay()
@@ -705,7 +722,7 @@ def run_ours(args, ws, rank, local):
     # toed_detect_host_batch: page-locked host images in, host edgel lists
     # out; the copy engine brings the images in over E2E_CHUNKS groups while
     # one detection launch runs (its CTAs wait for their group's copy), and
-    # the ordering pass writes the lists into host memory
+    # the edgel kernel copies each list into host memory as its bands finish
     h_imgs = [torch.as_tensor(im).pin_memory() for im in images]
     h_outs = det.alloc_host_outputs([im.shape for im in images], None, toed.TOED_F32, index=False)
     for o, c in zip(h_outs, caps):
@@ -750,14 +767,6 @@ def run_ours(args, ws, rank, local):
     fl = flops_per_px(r) * npx
     achieved = fl / (kernel_ms * 1e-3) / 1e12
     rho = n_edgels / npx
-    bytes_alg = npx * 4 + n_edgels * 16 + 4 * len(images)
-    hbm_ach = bytes_alg / (kernel_ms * 1e-3) / 1e9
-    # DRAM bytes of one launch from the committed ncu summary, scaled by pixels
-    traffic = None
-    tf = os.path.join(ROOT, "profiles", "toed_detect_kernel__uneven_batch64_sigma1.5.traffic.txt")
-    if os.path.exists(tf):
-        kv = dict(line.split() for line in open(tf) if line.strip() and not line.startswith("#"))
-        traffic = int(int(kv["dram_bytes_per_launch"]) * npx / int(kv["pixels"]))
 
     value = ws * npx / (ms * 1e-3) / 1e6
     line = {
@@ -779,13 +788,10 @@ def run_ours(args, ws, rank, local):
                 # host memory and the C2C link are shared with the machine's other jobs
                 "step_ms": {"mean": round(e2e_ms, 4), "median": round(float(np.median(e2e_steps)), 4),
                             "min": round(min(e2e_steps), 4), "max": round(max(e2e_steps), 4)}},
-        # the contract's roofline is HBM (algorithmic bytes vs the measured
-        # copy bandwidth); this stencil's binding roof is FP32 issue, given
+        # the contract's roofline is HBM (the step's algorithmic bytes vs the
+        # measured copy bandwidth); this stencil's binding roof is FP32 issue, given
         # beside it against the FP32 FMA rate measured in this process
-        "roofline": {"bound": "hbm", "achieved": round(hbm_ach, 2), "peak": hbm_peak, "unit": "GB/s",
-                     "frac": round(hbm_ach / hbm_peak, 5), "traffic": traffic,
-                     "bytes_per_px": round(bytes_alg / npx, 4),
-                     "traffic_bytes_per_px": round(traffic / npx, 3) if traffic else None,
+        "roofline": {**hbm_roofline(npx, n_edgels, len(images), ms, hbm_peak),
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6.8 TB/s",
                      "fp32": {"achieved": round(achieved, 3), "peak": round(fp32_peak, 3), "unit": "TFLOP/s",
                               "frac": round(achieved / fp32_peak, 4), "flops_per_px": flops_per_px(r),
