@@ -1134,6 +1134,7 @@ extern "C" toed_status toed_subpix_to_correct_batch(toed_ctx* c, const toed_edge
             s.img_count = c->img_count;
             s.keep = c->keep;
             s.work = c->sp_work;
+            s.num_sms = c->num_sms;
             cudaError_t e = subpix_launch(mp, cn, prm, r, s, stream);
             if (e != cudaSuccess) {
                 g_last_cuda_error = std::string("subpix_launch: ") + cudaGetErrorString(e);

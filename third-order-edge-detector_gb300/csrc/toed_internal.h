@@ -59,6 +59,7 @@ struct SubScratch {
     int* img_count;       // per map
     unsigned char* keep;  // per staged edgel
     double* work;         // interp_n > 0: resized maps (and orientations), per work pixel
+    int num_sms;
 };
 
 // Enqueue the TO-correction kernels for up to kBatchMax maps (toed_subpix.cu).

@@ -1459,8 +1459,8 @@ cudaError_t subpix_launch(const toed_edgemap* maps, int n, const toed_subpix_par
     // few tiles of segments are shared out, each over several CTAs, until some four
     // CTAs an SM have work: the FP64 distance tests of 22 tiles (two 501 x 667
     // work grids) kept 22 SMs busy, 107 us against 45 shared out eight ways.  From
-    // 305 tiles on a CTA takes a whole one (1024 tiles: 110 us)
-    const unsigned shares = (unsigned)std::min(8, std::max(1, 608 / p->n_seg_tiles));
+    // two an SM on (305 of 152) a CTA takes a whole one (1024 tiles: 110 us)
+    const unsigned shares = (unsigned)std::min(8, std::max(1, 4 * s.num_sms / p->n_seg_tiles));
     if (e == cudaSuccess) e = cudaLaunchKernel((const void*)tc_isolate, dim3(p->n_seg_tiles, shares), dim3(256), args, 0, stream);
     size_t smem = 0;
     const void* cf = correct_entry(r, &smem);
