@@ -231,7 +231,8 @@ toed_status toed_detect_noalloc(const toed_image* image, const toed_params* para
  * :415-441) for a whole batch, pipelined: the batch is cut into `chunks`
  * groups of consecutive images, growing in pixel count, and the copy of
  * group k+1 to the device overlaps the detection of group k.  Page-locked
- * images, at most 64: one detection launch for the whole batch whose CTAs
+ * images, at most 64: one detection launch for the whole batch (two for 32
+ * float32 images or more of 56 Mpixel together, radius 6 at most) whose CTAs
  * wait (bounded) for their group's copy, which the call enqueues right after
  * the launch -- another host thread that waits for the whole device in that
  * moment (cudaDeviceSynchronize, cudaFree) can hold those copies back until

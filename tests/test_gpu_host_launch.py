@@ -1,6 +1,6 @@
-"""Host batches: one detection launch for a batch of up to 64 page-locked
-images, whatever its size (so the shape tuned for such a batch serves it);
-every layout of outputs, images without edgels and a lost copy in large batches."""
+"""Host batches of page-locked images: one detection launch, or two where the
+rule says so; every layout of outputs, images without edgels and lost copies in
+large batches; one group asked for; no device memory for the pixels."""
 import os
 import subprocess
 import sys
@@ -25,6 +25,84 @@ def _batch(synth, sizes):
 # 26.8 Mpixel, the larger part behind the first half; sizes uneven, one image empty
 SIZES = [(1500, 1400), (900, 2100), (2011, 1301), (1400, 1500), (2048, 2048), (1203, 907), (2048, 2048), (1801, 2001), (640, 1111),
          (1500, 1400)]
+
+
+# 57.6 Mpixel in 35 images, uneven, one of the first and one of the second part empty (see MANY_EMPTY)
+MANY = [(1100 + 37 * (k % 7), 1300 + 29 * (k % 5)) for k in range(35)]
+MANY_EMPTY = (3, 30)
+
+
+def _many(synth):
+    out = _batch(synth, MANY)
+    out[30] = torch.full(MANY[30], 55.0).pin_memory()
+    return out
+
+
+@pytest.mark.parametrize("pin", [True, False])
+@pytest.mark.parametrize("f64", [False, True])
+def test_two_launches_for_many_images(toed, synth, pin, f64):
+    """At the rule's lines: 35 float32 images of 57.6 Mpixel take two launches,
+    31 of them, a wider filter or less than 56 Mpixel one; the lists are the
+    device batch's, also at a shape tuned for the whole batch."""
+    det = toed.Detector(0)
+    host = _many(synth)
+    assert sum(im.numel() for im in host) > 56e6
+    dt = toed.TOED_F64 if f64 else toed.TOED_F32
+    outs = det.alloc_host_outputs(MANY, capacity=200_000, out_dtype=dt, index=True, pin=pin)
+
+    def launches(n, sigma, images=None):
+        images = images or host[:n]
+        det.profile_begin()
+        det.detect_host(images, outs[:n], toed.make_params(sigma, 0, 2.0, 10, dt))
+        return det.profile_end()[1]
+
+    def same(n, sigma):
+        ref = det.detect_batch([im.cuda() for im in host[:n]], sigma=sigma, out_dtype=dt)
+        for k, (r, o) in enumerate(zip(ref, outs)):
+            m = int(o["count"].item())
+            assert m == r["count"] and (m == 0 if k in MANY_EMPTY else m > 1000)
+            assert torch.equal(o["edgels"][:m], r["edgels"].cpu())
+            assert torch.equal(o["index"][:m], r["index"].cpu())
+
+    assert launches(35, 1.5) == 2
+    same(35, 1.5)
+    assert launches(35, 1.0) == 2
+    same(35, 1.0)
+    assert launches(31, 1.5) == 1 and launches(33, 1.5) == 1 and launches(35, 1.6) == 1
+    same(35, 1.6)
+    small = [im[:, 200:].contiguous().pin_memory() for im in host]
+    assert launches(35, 1.5, [im.round().to(torch.uint8).pin_memory() for im in host]) == 1
+    assert sum(im.numel() for im in small) < 56e6 and launches(35, 1.5, small) == 1
+    for rows, staging in ((62, "plain"), (510, "tma")):
+        det.set_tuning(toed.make_params(1.5), rows, staging)
+        assert launches(35, 1.5) == 2
+        same(35, 1.5)
+
+
+@pytest.mark.parametrize("group", [2, 31])
+def test_lost_copy_in_either_part(toed, group):
+    """A ready flag of the first, or the second, of two launches is withheld."""
+    _child(f"""
+from test_gpu_host_launch import MANY, _many
+host = _many(synth)
+ref = [r["count"] for r in det.detect_batch([im.cuda() for im in host], sigma=1.5)]
+outs = det.alloc_host_outputs(MANY, capacity=200000)
+os.environ["TOED_TEST_WITHHOLD_READY"] = "{group}"
+os.environ["TOED_TEST_READY_SPINS"] = "20000"
+t0 = time.time()
+try:
+    det.detect_host(host, outs, prm)
+    raise SystemExit("no time-out")
+except toed.ToedError as e:
+    assert e.status == toed.TOED_ERR_TIMEOUT, e
+assert time.time() - t0 < 5
+got = [int(o["count"].item()) for o in outs]
+assert got[:{group}] == ref[:{group}] and got[{group}] == 0, (got, ref)
+del os.environ["TOED_TEST_WITHHOLD_READY"], os.environ["TOED_TEST_READY_SPINS"]
+det.detect_host(host, outs, prm)
+assert [int(o["count"].item()) for o in outs] == ref
+print("OK")
+""")
 
 
 @pytest.mark.parametrize("pin", [True, False])

@@ -417,6 +417,14 @@ static int plan_ed_rows(const toed_image* images, int n, int num_sms)
     return t;
 }
 
+// Strip rows at most of a launch that waits for its pixels: units this short
+// leave little to do once the last image is in.  Host batches, sigma 1.5, the
+// heights of plan_strip_rows / 254 / 126 / 62 rows, us a call: 64 uneven images
+// 2486 / 2422 / 2414 / 2406, eight 2048 x 2048 1117 / 1087 / 1038 / 1042, 36 of
+// 1080 x 1920 2292 / 2146 / 2137 / 2119, 16 of 1024 x 1024 619 / 621 / 603 / 598;
+// at sigma 3 62 rows' halos begin to show.
+constexpr int kWaitStripRows = 126;
+
 // One list's mapped host buffers (toed_detect_host_batch).
 struct HostList {
     void* edgels;
@@ -468,6 +476,7 @@ static toed_status detect_chunk(toed_ctx* c, const toed_image* images, int n, co
     p->thr2 = prm->threshold < 0.f ? -1.f : prm->threshold * prm->threshold * 0.9999f;
     p->border = prm->border;
     p->S = use ? use->strip_rows : plan_strip_rows(images, n, resident);
+    if (wait_slot) p->S = std::min(p->S, kWaitStripRows);
     p->n_img = n;
     p->out_f64 = (prm->out_dtype == TOED_F64) ? 1 : 0;
     p->radius = r;
@@ -600,12 +609,12 @@ static toed_status check_batch(const toed_ctx* c, const toed_image* images, int 
 // The batch in chunks of kBatchMax images (caller holds c->mu, device set).
 static toed_status detect_all(toed_ctx* c, const toed_image* images, int n, const toed_params* prm,
                               cudaStream_t stream, const toed_tuning* force = nullptr, const int* wait_slot = nullptr,
-                              const HostList* hosts = nullptr, bool in_place = false)
+                              const HostList* hosts = nullptr, bool in_place = false, bool first = true)
 {
     const int r = radius_of(prm);
     toed_status st = TOED_OK;
     for (int i0 = 0; i0 < n && st == TOED_OK; i0 += kBatchMax)
-        st = detect_chunk(c, images + i0, std::min(kBatchMax, n - i0), prm, r, i0 == 0, stream, force,
+        st = detect_chunk(c, images + i0, std::min(kBatchMax, n - i0), prm, r, first && i0 == 0, stream, force,
                           wait_slot ? wait_slot + i0 : nullptr, hosts ? hosts + i0 : nullptr, in_place);
     return st;
 }
@@ -715,6 +724,33 @@ extern "C" toed_status toed_detect(toed_ctx* c, const toed_image* image, const t
     return toed_detect_batch(c, image, 1, prm, stream);
 }
 
+// Images of the first of two pipelines that a batch of page-locked images runs
+// as, or n: one.  The first part's scan, edgels and lists then hide in the wait
+// for the second part's pixels, if there is one: where the link is the bound
+// (float32 pixels and radius 6 at most; 22 us a Mpixel over the link, 21 in the
+// kernels at radius 6), and enough images that neither part waits for a few large
+// ones.  One and two launches, us a call at sigma 1.5: 64 uneven images, 79
+// Mpixel, 2414 / 2263 (another 2717 / 2558); 64 of 1080 x 1920 3703 / 3557; 64, 56
+// of 1024 x 1024 2028 / 1951, 1807 / 1747; 48 uneven, 59 Mpixel, 1817 / 1736; 36 of
+// 1080 x 1920 2137 / 2113.  Beyond the lines: 28 of 1080 x 1920 1703 / 1724, 14 of
+// 2048 x 2048 1685 / 1736, three 8K 3207 / 3293, eight 2048 x 2048 1038 / 1121; 64
+// of 1080 x 1920 at sigma 2 4054 / 4088; 64 uneven 8-bit images 2296 / 2364.
+// Cuts at 55 and 70 % gain less (2340, 2415 on the first).
+constexpr int kTwoImages = 32, kTwoRadius = 6, kTwoPercent = 40;
+constexpr long long kTwoPixels = 56000000;
+static int first_part(const toed_host_image* images, int n, long long total_px, int r)
+{
+    if (n < kTwoImages || r > kTwoRadius || total_px < kTwoPixels) return n;
+    for (int i = 0; i < n; ++i)
+        if (images[i].dtype != TOED_F32) return n;
+    long long px = 0;
+    for (int i = 0; i + 1 < n; ++i) {
+        px += (long long)images[i].height * images[i].width;
+        if (px * 100 >= total_px * kTwoPercent) return i + 1;
+    }
+    return n;
+}
+
 // Launches run one at a time, each waited for: CUDA_LAUNCH_BLOCKING=1, or a
 // tool injected into the runtime (profilers and checkers serialise work).
 // (Nsight Compute marks its target process with NV_NSIGHT_INJECTION_* and
@@ -805,7 +841,7 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
         return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
     };
     // Page-locked inputs: the copy engine brings the groups into device memory
-    // while ONE detection launch runs, each image's CTAs waiting (bounded) for
+    // while one detection launch, or two, run, each image's CTAs waiting (bounded) for
     // its group's ready flag, which the copy engine writes after the group's
     // pixels -- every pixel crosses the link once and no group boundary
     // drains the GPU.  Pageable inputs: staged copies per group, one
@@ -833,8 +869,9 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
     if (inplace) chunks = 1;
     std::vector<cudaEvent_t> ev_in(chunks, nullptr), ev_det(chunks, nullptr);
     std::vector<int> first(chunks + 1, n);
-    // (flagged: one launch of at most kBatchMax images, so that nothing between
-    // the launch and the copies' enqueueing can wait for the device; never
+    // (flagged: one launch of at most kBatchMax images, or two whose scratch is
+    // there, so that nothing between the launch and the copies' enqueueing can
+    // wait for the device; never
     // when launches run serialised -- CUDA_LAUNCH_BLOCKING, or a profiler or
     // checker injected into the runtime -- since then the waiting launch
     // would hold the host or the device until its wait gives up)
@@ -955,7 +992,28 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
         const int early = std::min(chunks, 2);
         for (int k = 0; k < early; ++k) TOED_HB(enqueue_group(k));
         TOED_HB(preload_finalize(radius_of(prm), prm->orientation == TOED_ORI_QAD));
-        st = detect_all(c, dev.data(), n, prm, stream, nullptr, slot.data(), direct ? lists.data() : nullptr);
+        // (the shape tuned for the whole batch serves both parts)
+        const toed_tuning& whole =
+            c->tune[radius_of(prm)][prm->precision != TOED_FP32 ? 1 : 0][size_class(dev.data(), n)];
+        const toed_tuning* shape = whole.strip_rows > 0 ? &whole : nullptr;
+        const HostList* hl = direct ? lists.data() : nullptr;
+        const int cut = first_part(images, n, total_px, radius_of(prm));
+        if (cut < n) {
+            // the scratch of both is grown before the first launch: growing waits for the device
+            long long segs = 0, bands = 0, cap = 0;
+            for (int i = 0; i < n; ++i) {
+                const long long nseg = 2LL * images[i].height * ((images[i].width + kInner - 1) / kInner);
+                segs += (nseg + kScanTileMax - 1) / kScanTileMax * kScanTileMax;
+                bands += images[i].height;
+                cap += images[i].capacity;
+            }
+            st = ensure_scratch(c, staging_records(cap, most_warps(c)), segs, segs / kSegTile, stream);
+            if (st == TOED_OK && direct) st = grow(&c->band, &c->band_cap, bands, stream);
+        }
+        if (st == TOED_OK) st = detect_all(c, dev.data(), cut, prm, stream, shape, slot.data(), hl);
+        if (st == TOED_OK && cut < n)
+            st = detect_all(c, dev.data() + cut, n - cut, prm, stream, shape, slot.data() + cut, hl ? hl + cut : nullptr,
+                            false, false);
         c->ready_spins = kReadySpinLimit;
         if (st != TOED_OK) return fail(st);
         TOED_HB(cudaMemcpyAsync(c->hb_cnt + n, c->words + 2, sizeof(int), cudaMemcpyDeviceToDevice, stream));
