@@ -136,7 +136,7 @@ toed_status toed_destroy(toed_ctx* ctx);
 toed_status toed_reserve(toed_ctx* ctx, long long max_pixels, long long max_edgels, int max_images);
 
 /* Fused detection of one image / a batch of images of any sizes in one
- * persistent launch (plus a short ordering pass).  Asynchronous on
+ * persistent launch (plus a scan and the edgel kernel).  Asynchronous on
  * `stream`; graph-capturable once scratch is reserved. */
 toed_status toed_detect(toed_ctx* ctx, const toed_image* image, const toed_params* params,
                         cudaStream_t stream);
@@ -293,7 +293,8 @@ toed_status toed_write_edgels_txt(const char* path, const void* edgels, int dtyp
 typedef struct toed_tuning {
     int strip_rows;  /* 16k - 2 for k in 1, 2, 4, ..., 64 */
     int staging;     /* input row staging: 1 TMA (float32 images whose rows are 16-byte aligned),
-                        0 or 2 loads prefetched a step ahead in registers */
+                        0 loads prefetched a step ahead in registers (2: the same, kept for
+                        callers of the former asynchronous copies) */
     float ms;        /* measured time of one detection of the batch (autotune output) */
 } toed_tuning;
 

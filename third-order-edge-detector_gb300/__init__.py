@@ -371,8 +371,8 @@ class Detector:
 
     def set_tuning(self, params: toed_params, strip_rows=None, staging="tma"):
         """Install a launch shape (strip_rows None: the built-in heuristic);
-        staging: "tma", or "async" / "plain" for loads (True / False mean "tma" /
-        "plain")."""
+        staging: "tma", or "plain" for loads (True / False mean these; "async",
+        the former asynchronous copies, is "plain")."""
         if isinstance(staging, bool):
             staging = "tma" if staging else "plain"
         t = toed_tuning(int(strip_rows), _STAGING_NAMES.index(staging), 0.0) if strip_rows is not None else None
@@ -414,7 +414,7 @@ class Detector:
 
     def capture(self, images, outs, params: toed_params, warmup: int = 1):
         """Capture detect_into(images, outs, params) in a CUDA graph (the
-        persistent detection launch plus the ordering pass) and return it;
+        detection, scan and edgel launches) and return it;
         ``graph.replay()`` re-runs the batch on the same buffers with no host
         work.  Scratch is reserved first, so nothing allocates under capture."""
         t = self.torch

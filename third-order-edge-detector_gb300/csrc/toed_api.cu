@@ -118,8 +118,8 @@ void encode_rows_map(CUtensorMap* m, DetImage& d, int r)
 
 using namespace toed;
 
-// NVTX range over one phase of a call (the detection launch, the ordering
-// pass, a copy group, ...): no cost unless a profiler is attached.
+// NVTX range over one phase of a call (the detection launch, scan and edgels,
+// a copy group, ...): no cost unless a profiler is attached.
 struct NvtxRange {
     explicit NvtxRange(const char* name) { nvtxRangePushA(name); }
     ~NvtxRange() { nvtxRangePop(); }
@@ -579,7 +579,7 @@ static toed_status detect_chunk(toed_ctx* c, const toed_image* images, int n, co
     }
     if (ev1) TOED_CU(cudaEventRecord(ev1, stream));
     {
-        NvtxRange r("toed: ordering pass");
+        NvtxRange r("toed: scan and edgels");
         TOED_CU(launch_finalize(*p, stream));
     }
     return TOED_OK;
@@ -830,8 +830,8 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
     } while (0)
     // Page-locked host outputs are written by the edgel kernel as bands of a
     // list are complete, through their mapping into the device's address space
-    // (coherent over the C2C link): no count read-back and no copy per list.  Otherwise lists are copied back per group once its counts are
-    // known.
+    // (coherent over the C2C link): no count read-back and no copy per list.
+    // Otherwise lists are copied back per group once its counts are known.
     auto mapped = [](void* hp) -> void* {
         cudaPointerAttributes a;
         if (!hp || cudaPointerGetAttributes(&a, hp) != cudaSuccess) {

@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<R, NMSTO>::MINB)
             __syncthreads();
             if (!in) {
                 // the copy never arrived: the unit finds no edgels (its row
-                // segments are written empty, so the ordering pass reads no
+                // segments are written empty, so the scan reads no
                 // stale entries) and the call reports TOED_ERR_TIMEOUT
                 for (int i = tid; i < 2 * S_act; i += kThreads)
                     if (TOED_IN_BOUNDS(im.seg_base + (long long)(2 * ys + i) * im.nsc + sc < p.sc.seg_cap, p.sc.words))

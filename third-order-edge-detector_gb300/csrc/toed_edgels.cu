@@ -6,10 +6,10 @@
 //                p.seg_tile consecutive segments -- (2x-grid row, strip column)
 //                pairs, row-major per image -- and one CTA's work: it scans
 //                its counts and adds the sum of the image's earlier tiles,
-//                which every tile publishes as soon as it has its own (a
-//                chained scan with look-back: tiles are taken in order by a
-//                ticket, so every earlier tile is running or done, and the
-//                bounded wait ends);
+//                which every tile publishes as soon as it has its own (the
+//                single-pass scan with decoupled look-back of Merrill and
+//                Garland, 2016: tiles are taken in order by a ticket, so every
+//                earlier tile is running or done, and the bounded wait ends);
 //   fin_edgels   the edgels themselves.  A CTA takes the segments of one strip
 //                column over p.ed_rows image rows and stages the pixels that
 //                their windows cover in shared memory once; then a thread per

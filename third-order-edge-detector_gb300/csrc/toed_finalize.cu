@@ -10,7 +10,7 @@
 //   fin_scatter   : per tile, scan the segment counts, then copy the tile's
 //                   staged records cooperatively to their list positions
 //                   (global prefix - image base), converting to the output
-//                   dtype (the quick-and-dirty mode: toed_qad.cu).
+//                   dtype.
 #include "toed_common.cuh"
 #include "toed_internal.h"
 

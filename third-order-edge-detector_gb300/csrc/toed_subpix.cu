@@ -1084,8 +1084,9 @@ __global__ void __launch_bounds__(256) tc_isolate(const __grid_constant__ SubPar
     __syncthreads();
     const bool all = !(p.nbr > 0.0) || p.img_count[k] < 2;  // :567-568
     const double r2 = p.nbr * p.nbr;
-    // an edgel lies within sqrt(2) work pixels of its own; search the id map
-    // (work grid) around it, compare in original pixels as the reference does
+    // the max test keeps an edgel within half a work pixel an axis of its own, so
+    // two within the radius have pixels at most that and one apart; search the id
+    // map (work grid) so far around, compare in original pixels as the reference does
     const int reach = (int)ceil(p.nbr * M.scale + 1.5);
     for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < total; e += gridDim.y * blockDim.x) {
         int lo = 0, hi = kSegTile - 1;  // last segment with s_dst <= e
@@ -1166,7 +1167,8 @@ __global__ void __launch_bounds__(256) tc_compact(const __grid_constant__ SubPar
 }
 
 // Dense TO_E / TO_O (:708-715) at interp_n = 0, one pass: an edgel lies within
-// sqrt(2) of its pixel, so it rounds onto it or one of the eight around, and
+// half a pixel an axis of its own (sqrt(2) whatever the fit's rounding), so it
+// rounds onto it or one of the eight around, and
 // the edgel that a pixel gets -- the last in list order, row-major by pixel --
 // is the last of the tile's and its neighbours' pixels, in row-major order,
 // whose edgel rounds onto it: a vote in shared memory.  Every pixel
@@ -1472,7 +1474,7 @@ cudaError_t subpix_launch(const toed_edgemap* maps, int n, const toed_subpix_par
     if (dense && sc == 1 && e == cudaSuccess)
         e = cudaLaunchKernel((const void*)tc_dense_gather, dim3(tiles), dim3(256), args, 0, stream);
     if (e == cudaSuccess) e = cudaLaunchKernel((const void*)tc_compact, dim3(p->n_seg_tiles), dim3(256), args, 0, stream);
-    // ordering pass shared with the detector
+    // the ordering pass (toed_finalize.cu)
     BatchParams* b = new BatchParams();
     std::memset(b, 0, sizeof(BatchParams));
     std::unique_ptr<BatchParams> bguard(b);
