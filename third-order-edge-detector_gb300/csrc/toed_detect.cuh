@@ -434,9 +434,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<R, NMSTO>::MINB)
     __syncthreads();
     int bi = 0;             // buffer of the next box to arrive by TMA
     uint32_t phase = 0;     // its mbarrier's phase
-    // not 0 once a wait for a box gave up: 32, the box's phase (bit 0), buffer
-    // (bits 1, 2) and, in thread 0, the boxes then in flight (bits 3, 4)
-    int dead = 0;
+    bool dead = false;      // a wait for a box gave up
     int slot = 0;           // of sScal that holds the unit
 
     for (;;) {
@@ -539,8 +537,18 @@ __global__ void __launch_bounds__(kThreads, Cfg<R, NMSTO>::MINB)
                 float* box = sRaw + bi * (B * C::BW);
                 if (tma) {
                     if (!dead && !mbar_wait(bar + 8 * bi, phase)) {
-                        dead = 32 | ((issued - q) & 3) << 3 | bi << 1 | (int)phase;
+                        dead = true;
                         atomicOr(&p.sc.words[2], TOED_FLAG_TIMEOUT);
+                        // once more for what is in flight, nothing of which may outlive
+                        // the CTA's memory (thread 0 requests no more boxes)
+                        if (tid == 0)
+                            for (int k = q, b = bi, ph = phase; k < issued; ++k) {
+                                mbar_wait(bar + 8 * b, ph);
+                                if (++b == C::NBUF) {
+                                    b = 0;
+                                    ph ^= 1;
+                                }
+                            }
                     }
                 } else {
                     __syncwarp();
@@ -720,16 +728,6 @@ __global__ void __launch_bounds__(kThreads, Cfg<R, NMSTO>::MINB)
             rb = ring_wrap<C::RING>(rb + B);
         }
     }
-    // nothing may be in flight towards an exited CTA's memory: the boxes that
-    // thread 0 had requested when its wait gave up (it requests none after that)
-    if (dead && tid == 0)
-        for (int k = 0, q = (dead >> 1) & 3, ph = dead & 1; k < ((dead >> 3) & 3); ++k) {
-            mbar_wait(bar + 8 * q, ph);
-            if (++q == C::NBUF) {
-                q = 0;
-                ph ^= 1;
-            }
-        }
 }
 
 }  // namespace toed

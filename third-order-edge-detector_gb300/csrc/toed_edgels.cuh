@@ -538,7 +538,6 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
         }
     }
     const long long cap = im.cap;
-    bool late = false;  // the wait for the pixels gave up
     for (int c0 = 0; c0 < total; c0 += kEdChunk) {
         // the chunk's edgels, then their records ordered by 2x column parity
         for (int u = 0, at = run - c0; u < 2; ++u)
@@ -547,8 +546,10 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
         sPos[tid] = -1;
         if (tid == 0) sFlags = 0;
         __syncthreads();
-        if (im.tma && c0 == 0) late = !mbar_wait(bar, 0);
-        if (late && tid == 0) atomicOr(&p.sc.words[2], TOED_FLAG_TIMEOUT);
+        if (im.tma && c0 == 0 && !mbar_wait(bar, 0) && tid == 0) {
+            atomicOr(&p.sc.words[2], TOED_FLAG_TIMEOUT);
+            mbar_wait(bar, 0);  // once more: nothing may be in flight towards an exited CTA's memory
+        }
         const int n = min(kEdChunk, total - c0);
         Staged e = {};
         int pos = -1;
@@ -669,7 +670,6 @@ __global__ void __launch_bounds__(kEdThreads, R <= 8 && !QAD ? 3 : 2) fin_edgels
         __syncthreads();  // the next chunk overwrites the lists
     }
     if (im.host_out) band_done(p, im, ty, s_warp);
-    if (late && tid == 0) mbar_wait(bar, 0);  // nothing may be in flight towards an exited CTA's memory
 }
 
 struct EdEntry {
