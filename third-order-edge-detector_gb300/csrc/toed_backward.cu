@@ -711,7 +711,12 @@ __global__ void __launch_bounds__(kBwAdjThreads, BwCfg<R>::MINB) bw_adjoint(cons
             // added at the end: the sums' rounding is then relative to the
             // window's contrast, not to its brightness
             // (8-bit pixels carry 2^23, the float whose last bits they are)
-            const float mid = by_warp ? 0.f : pix(im, rho >> 1, kap >> 1), zero = u8 ? 8388608.f : 0.f, less = zero + mid;
+            // -- not a number where the window needs a group that is not copied, so
+            // that all its values are none and count as ill-conditioned
+            const float mid = by_warp ? 0.f
+                              : window_cut(wy, wx, NU, im.H, im.W, skew, span) ? __int_as_float(0x7fc00000)
+                                                                               : pix(im, rho >> 1, kap >> 1);
+            const float zero = u8 ? 8388608.f : 0.f, less = zero + mid;
             BwValues o = {};
             __syncwarp();
             if (!by_warp) stage(0, 0);
@@ -795,9 +800,8 @@ __global__ void __launch_bounds__(kBwAdjThreads, BwCfg<R>::MINB) bw_adjoint(cons
                 for (int q = 0; q < 4; ++q) go[q] = g[q];
             }
             const bool used = go[0] != 0.f || go[1] != 0.f || go[2] != 0.f || go[3] != 0.f;
-            // (pixel by pixel too: windows over a group that is not copied)
-            unsigned ill = __ballot_sync(0xffffffffu, lane < nw && (by_warp || window_cut(wy, wx, NU, im.H, im.W, skew, span) ||
-                                                                    ill_conditioned(o, nv, xmaj, used, p.ill_curve)));
+            unsigned ill = __ballot_sync(0xffffffffu,
+                                         lane < nw && (by_warp || ill_conditioned(o, nv, xmaj, used, p.ill_curve)));
             for (; ill; ill &= ill - 1) {
                 const int w = __ffs(ill) - 1;
                 const int bits = eval_edgel_warp<R>(im, __shfl_sync(0xffffffffu, rho, w), __shfl_sync(0xffffffffu, kap, w),
