@@ -721,7 +721,7 @@ def run_ours(args, ws, rank, local):
     # ---- end to end through the public API with host buffers -----------
     # toed_detect_host_batch: page-locked host images in, host edgel lists
     # out; the copy engine brings the images in over E2E_CHUNKS groups while
-    # one detection launch runs (its CTAs wait for their group's copy), and
+    # two detection launches run (their CTAs wait for their group's copy), and
     # the edgel kernel copies each list into host memory as its bands finish
     h_imgs = [torch.as_tensor(im).pin_memory() for im in images]
     h_outs = det.alloc_host_outputs([im.shape for im in images], None, toed.TOED_F32, index=False)

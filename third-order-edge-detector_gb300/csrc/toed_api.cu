@@ -854,9 +854,10 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
     }
     // Asked for one group, page-locked images still cross in several: one group
     // leaves nothing to overlap (64 images, 79 Mpixel: 3.70 ms a call, 2.49 with
-    // an image a group), and the lists are the same.  Beyond one launch's images
-    // a group costs launches of its own.
-    if (zin && chunks <= 1) chunks = n <= kBatchMax ? n : 4;
+    // an image a group), and the lists are the same.  Where a group costs launches
+    // of its own, four.
+    const bool one_call = n <= kBatchMax && !launches_serialised();
+    if (zin && chunks <= 1) chunks = one_call ? n : 4;
     chunks = std::max(1, std::min(chunks, n));
     // Page-locked images that device memory has no room for are read in place
     // through their mapping (by loads, and twice over the link: 6.5 ms).
@@ -875,7 +876,7 @@ extern "C" toed_status toed_detect_host_batch(toed_ctx* c, const toed_host_image
     // when launches run serialised -- CUDA_LAUNCH_BLOCKING, or a profiler or
     // checker injected into the runtime -- since then the waiting launch
     // would hold the host or the device until its wait gives up)
-    const bool flagged = zin && !inplace && n <= kBatchMax && !launches_serialised();
+    const bool flagged = zin && !inplace && one_call;
     if (flagged) {
         const long long had = c->hb_ready_cap;
         if ((st = grow(&c->hb_ready, &c->hb_ready_cap, (long long)chunks, stream)) != TOED_OK) return fail(st);
